@@ -2,6 +2,10 @@
 // basis and the variational energy E = sum_i c_i sigma_i
 // (compute_variational_energy, local_conn.cpp:148-229).
 //
+// Large bases are matched by string groups (contract_strings, vvstr.cu); the
+// others, and those the groups do not take (64 orbitals, duplicates, mixed
+// electron counts), by the walk here.
+//
 // Same warp-per-row walk as the builder; hits in the basis are accumulated
 // per lane with Dot2 (TwoProduct + TwoSum) and merged across the warp, and
 // the row energies are summed with Dot2 again, so the result carries about
@@ -13,6 +17,8 @@ namespace dnq {
 
 void check_orbitals(const u64* d, i64 n, int n_orb, cudaStream_t s);
 void launch_diag(const dnq_ctx_s* c, const u64* d, i64 n, double* out, cudaStream_t s);
+bool contract_strings(dnq_ctx_s* ctx, const u64* V, i64 n, const double* cd, int n_orb,
+                      double single_thr, double cut, double* sigma, cudaStream_t s, double* e);
 
 namespace {
 
@@ -123,25 +129,74 @@ __global__ void k_final(const double* part, int nb, double* out) {
     *out = a.s + a.c;
 }
 
-__global__ void k_prefix(PairTableView T, i64 nrows, double cut, i64* plen) {
+// Prefix length of every table row for one cut; *kept sums them.
+__global__ void k_prefix(PairTableView T, i64 nrows, double cut, i64* plen,
+                         unsigned long long* kept) {
+    unsigned long long sum = 0;
     for (i64 r = blockIdx.x * (i64)blockDim.x + threadIdx.x; r < nrows;
          r += (i64)gridDim.x * blockDim.x) {
         const i64 lo = T.off[r], len = T.off[r + 1] - lo;
-        if (cut <= 0.0) { plen[r] = len; continue; }
-        i64 L = 0, R = len;
+        i64 L = 0, R = cut <= 0.0 ? 0 : len;
         while (L < R) {
             const i64 mid = L + (R - L) / 2;
             if (fabs(T.v[lo + mid]) >= cut) L = mid + 1; else R = mid;
         }
+        if (cut <= 0.0) L = len;
         plen[r] = L;
+        sum += L;
     }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(kept, sum);
 }
 
 }  // namespace
 
+// Whether the string groups contract faster than the candidate walk.  The
+// walk takes about 0.1 us per candidate of a row (a warp steps through 32 at
+// a time, a hash probe each) for every 2,500 rows, the groups 500 us more
+// than the walk's own fixed cost, most of it sorting and indexing the
+// basis.  Measured (walk / groups, us): 703 / 792 at 9.7e6 candidates (3,000
+// rows of 14 orbitals), 1,726 / 876 at 3.2e7, 51,633 / 1,714 at 1.35e9 (20,011
+// rows of 30 orbitals); 352 / 903 when a cut of 0.1 leaves few of 2.7e7.
+// kept = share of the doubles the cut keeps.
+bool contract_by_strings(i64 n, int n_orb, int na, int nb, double kept) {
+    const double va = n_orb - na, vb = n_orb - nb;
+    const double singles = na * va + nb * vb;
+    const double doubles = 0.25 * na * (na - 1.0) * va * (va - 1.0) +
+                           0.25 * nb * (nb - 1.0) * vb * (vb - 1.0) + na * va * nb * vb;
+    return (singles + kept * doubles) * std::max(1.0, (double)n / 2500.0) > 5000.0;
+}
+
 // sigma (optional) and E for a fixed basis; returns E on the host.
 double contract_energy(dnq_ctx_s* ctx, const u64* Vd, i64 n, const double* cd, int n_orb,
                        bool use_hb, double eps1, double* sigma, cudaStream_t s) {
+    const double single_thr = use_hb ? std::max(eps1, kElemThresh) : kElemThresh;   // :176-178
+    const double cut = use_hb ? hb_cutoff(ctx, eps1) : full_cutoff();
+    const PairTableView tab = ctx->view().tab;
+    DBuf<i64> plen(ctx->tab.n_rows, s);
+    DBuf<unsigned long long> kept(1, s);
+    DNQ_CUDA(cudaMemsetAsync(kept.p, 0, 8, s));
+    k_prefix<<<64, 256, 0, s>>>(tab, ctx->tab.n_rows, cut, plen.p, kept.p);
+    DNQ_CHECK_LAUNCH();
+    if (n_orb < 64 && !default_options().force_walk) {
+        u64 d0[2];
+        unsigned long long hk = 0;
+        DNQ_CUDA(cudaMemcpyAsync(d0, Vd, sizeof(d0), cudaMemcpyDeviceToHost, s));
+        DNQ_CUDA(cudaMemcpyAsync(&hk, kept.p, 8, cudaMemcpyDeviceToHost, s));
+        DNQ_CUDA(cudaStreamSynchronize(s));
+        if (contract_by_strings(n, n_orb, __builtin_popcountll(d0[0]),
+                                __builtin_popcountll(d0[1]),
+                                (double)hk / std::max<double>(1.0, (double)ctx->tab.n_entries))) {
+            try {
+                double e = 0.0;
+                if (contract_strings(ctx, Vd, n, cd, n_orb, single_thr, cut, sigma, s, &e))
+                    return e;
+            } catch (const Error& x) {   // the indices did not fit: the walk needs a map only
+                if (x.code != DNQ_ERR_OUT_OF_MEMORY) throw;
+            }
+        }
+    }
     DetMap map;
     build_detmap(map, Vd, n, false, s);
     DBuf<double> diag(n, s);
@@ -154,11 +209,8 @@ double contract_energy(dnq_ctx_s* ctx, const u64* Vd, i64 n, const double* cd, i
     P.coeff = cd;
     P.diag = diag.p;
     P.n_orb = n_orb;
-    P.single_thr = use_hb ? std::max(eps1, kElemThresh) : kElemThresh;   // :176-178
-    P.cut = use_hb ? hb_cutoff(ctx, eps1) : full_cutoff();
-    DBuf<i64> plen(ctx->tab.n_rows, s);
-    k_prefix<<<64, 256, 0, s>>>(P.C.tab, ctx->tab.n_rows, P.cut, plen.p);
-    DNQ_CHECK_LAUNCH();
+    P.single_thr = single_thr;
+    P.cut = cut;
     P.plen = plen.p;
     DBuf<int> next(1, s);
     DNQ_CUDA(cudaMemsetAsync(next.p, 0, 4, s));

@@ -536,6 +536,7 @@ struct VVParams {
     int policy;
     double eps1;
     double cut;             // doubles: keep w >= cut (and > 1e-15)
+    double single_thr;      // singles: keep |h| > single_thr
     const double* psi;
     u32 big_group;          // part C: binary search for groups longer than this
     int c_groupwalk;        // part C: short groups one at a time instead of packed
@@ -708,7 +709,7 @@ __device__ __forceinline__ bool keep_double(double cut, double h) {
 }
 
 __device__ __forceinline__ bool keep_single(const VVParams& P, double psr, double h) {
-    if (!(fabs(h) > kElemThresh)) return false;
+    if (!(fabs(h) > P.single_thr)) return false;
     if (P.policy == DNQ_POLICY_DYNAMIC) return fabs(h * psr) >= P.eps1;
     return true;
 }
@@ -967,10 +968,12 @@ __device__ __forceinline__ int small_div(int i, float rcp, int d, int& r) {
 // registers than passing them in).  gx and gy are the groups of x and y in
 // their indices (~0u: unknown); with the neighbour tables the groups of
 // their singles are read from the tables, else looked up by string.
-template <class W, class Q>
+// SL: only the rounds of slice sl of nsl (every nsl-th round of 32 singles).
+template <bool SL, class W, class Q>
 __device__ __forceinline__ void part_c(const VVParams& P, WarpShared& S, Q& q,
                                        unsigned long long& tests, bool bm, u64 a, u64 b, int na,
-                                       int nva, int nb, int nvb, u32 gx, u32 gy) {
+                                       int nva, int nb, int nvb, u32 gx, u32 gy, int sl = 0,
+                                       int nsl = 1) {
     const int lane = threadIdx.x & 31;
     const u64 x = bm ? b : a, y = bm ? a : b;
     const u8* occx = bm ? S.occb : S.occa;
@@ -990,13 +993,15 @@ __device__ __forceinline__ void part_c(const VVParams& P, WarpShared& S, Q& q,
     // neighbour-table row of x (its first entry; ~0: none), read one round ahead
     const u32 nrow = (bm ? P.b_nbr : P.a_nbr) && gx != 0xffffffffu
                          ? gx * (u32)nbr_stride(P.n_orb) : 0xffffffffu;
-    u32 gnext = nrow != 0xffffffffu && lane < nsx ? __ldg(&(bm ? P.b_nbr : P.a_nbr)[nrow + lane])
-                                                  : 0xffffffffu;
-    for (int s0 = 0; s0 < nsx; s0 += 32) {
+    const int first = SL ? 32 * sl : 0, step = SL ? 32 * nsl : 32;
+    u32 gnext = nrow != 0xffffffffu && first + lane < nsx
+                    ? __ldg(&(bm ? P.b_nbr : P.a_nbr)[nrow + first + lane])
+                    : 0xffffffffu;
+    for (int s0 = first; s0 < nsx; s0 += step) {
         const int sidx = s0 + lane;
         const u32 gcur = gnext;
-        if (nrow != 0xffffffffu && sidx + 32 < nsx)
-            gnext = __ldg(&(bm ? P.b_nbr : P.a_nbr)[nrow + sidx + 32]);
+        if (nrow != 0xffffffffu && sidx + step < nsx)
+            gnext = __ldg(&(bm ? P.b_nbr : P.a_nbr)[nrow + sidx + step]);
         u32 gs = 0, gl = 0, gg = 0xffffffffu;
         int hh = 0, pp = 0;
         if (sidx < nsx) {
@@ -1171,14 +1176,17 @@ __host__ __device__ __forceinline__ bool row_bm(uint4 ca, uint4 cb, int nsa, int
 // The members of row r = (a, b) in their fixed order: the diagonal, then
 // parts A, B and C.  q.push(hit, position, tag) is warp-collective, once
 // per step of 32; q.sync() follows every group of at most kScanU steps.
-template <class W, class Q>
+// SL: slice sl of nsl of the row -- its share of the members of parts A and B
+// and of part C's rounds; the diagonal belongs to slice 0.
+template <class W, bool SL = false, class Q>
 __device__ __forceinline__ void walk_row(const VVParams& P, int r, u64 a, u64 b, WarpShared& S,
-                                         Q& q, unsigned long long& tests) {
+                                         Q& q, unsigned long long& tests, int sl = 0,
+                                         int nsl = 1) {
     const int lane = threadIdx.x & 31;
     const W* ao = a_others<W>(P);
     const W aw = (W)a, bw = (W)b;
     const u64 all = low_mask(P.n_orb);
-    q.push(lane == 0, (u32)r, kHitD);
+    q.push(lane == 0 && (!SL || sl == 0), (u32)r, kHitD);
     // groups of parts A and B, looked up by lanes 0 and 1 side by side
     u32 st = 0, ln = 0;
     if (lane == 0 && !P.bmap.find(b, st, ln)) ln = 0;
@@ -1190,8 +1198,13 @@ __device__ __forceinline__ void walk_row(const VVParams& P, int r, u64 a, u64 b,
     // walk's speed depends on its code fitting the instruction cache
 #pragma unroll 1
     for (int part = 0; part < 2; ++part) {
-        const u32 gst = __shfl_sync(0xffffffffu, st, part);
-        const u32 gln = __shfl_sync(0xffffffffu, ln, part);
+        u32 gst = __shfl_sync(0xffffffffu, st, part);
+        u32 gln = __shfl_sync(0xffffffffu, ln, part);
+        if (SL) {
+            const u32 share = (gln + nsl - 1) / nsl, skip = min(gln, share * sl);
+            gst += skip;
+            gln = min(gln - skip, share);
+        }
         tests += gln;
         scan_same(q, part ? ao : b_others<W>(P), part ? bw : aw, gst, gln, part ? kHitB : kHitA);
     }
@@ -1221,8 +1234,9 @@ __device__ __forceinline__ void walk_row(const VVParams& P, int r, u64 a, u64 b,
     }
     // one call site for both directions: a second inlined copy of the walk
     // would not fit the instruction cache
-    part_c<W>(P, S, q, tests, bm, a, b, na, nva, nb, nvb,
-              __shfl_sync(0xffffffffu, grp, bm ? 0 : 1), __shfl_sync(0xffffffffu, grp, bm ? 1 : 0));
+    part_c<SL, W>(P, S, q, tests, bm, a, b, na, nva, nb, nvb,
+                  __shfl_sync(0xffffffffu, grp, bm ? 0 : 1),
+                  __shfl_sync(0xffffffffu, grp, bm ? 1 : 0), sl, nsl);
 }
 
 // A member's tag, given as a value or as a function read only on a hit.
@@ -2200,6 +2214,7 @@ VVParams make_params(dnq_ctx_s* ctx, const u64* V, i64 n, int n_orb, int policy,
     P.policy = policy;
     P.eps1 = eps1;
     P.cut = cut;
+    P.single_thr = kElemThresh;
     P.psi = psi;
     P.big_group = kBigGroup;
     P.c_groupwalk = opt.partc_groupwalk;
@@ -2505,7 +2520,241 @@ __global__ void k_sanitize(i64* rowptr, i64 n, i64 cap, const int* overflow, int
     for (i64 t = threadIdx.x; t <= n; t += blockDim.x) rowptr[t] = 0;
 }
 
+// ---------------------------------------------------------------------------
+// Matrix-free contraction sigma_i = sum_j H_ij c_j over a fixed basis and
+// E = sum_i c_i sigma_i (compute_variational_energy, local_conn.cpp:148-229)
+// from string groups: every ket that counts is a member of the basis, so the
+// members of a row are found as in the V->V build instead of probing every
+// candidate of the row in a hash.  Nothing is stored per member: the walk
+// evaluates them 32 at a time and each lane sums its products with Dot2.
+//
+// Bound: the walk's dependent L2 reads (group lookups, members, integrals).
+// A warp per row leaves the rows of the reference string as a tail (HF is
+// connected to most of a selected space), so a row is cut into up to one
+// slice per part C round, about kSliceTests tests each, and the slices'
+// sums are merged in order.  Whole call on 20,011 determinants of 30 orbitals
+// (1.35e9 candidates): 51.96 ms by the candidate walk, 1.72 ms here, most of
+// that the sorts and launches of the two indices.
+// ---------------------------------------------------------------------------
+constexpr u32 kSliceTests = 2048;        // tests per slice, few rows per warp
+constexpr u32 kSliceTestsMany = 1 << 17; // with many rows per warp only the longest are cut
+
+// Sets *mixed when the determinants differ in their electron counts (the
+// string tests count differing orbitals, which then says nothing of the
+// excitation rank).
+__global__ void k_mixed_counts(const u64* V, i64 n, u32* mixed) {
+    const int na = __popcll(V[0]), nb = __popcll(V[1]);
+    for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
+         t += (i64)gridDim.x * blockDim.x)
+        if (__popcll(V[2 * t]) != na || __popcll(V[2 * t + 1]) != nb) *mixed = 1u;
+}
+
+struct ContractOut {
+    const double* coeff;
+    DDb acc;
+    __device__ __forceinline__ void put(bool keep, u32 j, double h) {
+        if (keep) acc.add_prod(h, __ldg(&coeff[j]));
+    }
+};
+
+// Slices of the row at every place of the walk order (0: |c_i|^2 < 1e-12,
+// the row is skipped as in local_conn.cpp:188).
+__global__ void k_contract_slices(VVParams P, const u32* order, const double* coeff, u32 per,
+                                  u32* nsl) {
+    const u64 all = low_mask(P.n_orb);
+    for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t <= P.n;
+         t += (i64)gridDim.x * blockDim.x) {
+        if (t == P.n) {
+            nsl[t] = 0;   // the scan ends with the total
+            continue;
+        }
+        const u32 r = order[t];
+        const double ci = coeff[r];
+        if (ci * ci < 1e-12) {
+            nsl[t] = 0;
+            continue;
+        }
+        const u64 a = P.V[2 * (i64)r], b = P.V[2 * (i64)r + 1];
+        u32 sa = 0, la = 0, sb = 0, lb = 0;
+        u64 work = 0;
+        const int nsa = __popcll(a) * __popcll(~a & all), nsb = __popcll(b) * __popcll(~b & all);
+        int rounds = (nsa + 31) / 32;
+        if (P.amap.find(a, sa, la) && P.bmap.find(b, sb, lb)) {
+            const uint4 ca = P.a_cost[P.a_gid[sa]], cb = P.b_cost[P.b_gid[sb]];
+            const bool bm = row_bm(ca, cb, nsa, nsb);
+            if (bm) rounds = (nsb + 31) / 32;
+            work = (u64)la + lb + (bm ? cb.x + (u64)cb.y * ca.w + (u64)cb.z * (u32)nsa
+                                      : ca.x + (u64)ca.y * cb.w + (u64)ca.z * (u32)nsb);
+        }
+        const u64 want = 1 + work / per;
+        nsl[t] = (u32)max(1, (int)min((u64)rounds, want));
+    }
+}
+
+// (row, slice << 16 | slices) of every slice, in walk order.
+__global__ void k_contract_items(const u32* order, const u32* nsl, const i64* off, i64 n,
+                                 uint2* item) {
+    for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
+         t += (i64)gridDim.x * blockDim.x) {
+        const u32 k = nsl[t];
+        for (u32 q = 0; q < k; ++q) item[off[t] + q] = make_uint2(order[t], q << 16 | k);
+    }
+}
+
+template <class W>
+__global__ void __launch_bounds__(kWS * 32)
+k_contract_walk(VVParams P, const double* coeff, const uint2* item, i64 n_item, int* next,
+                double2* part) {
+    __shared__ WarpShared sh[kWS];
+    __shared__ HitRing rings[kWS];
+    WarpShared& S = sh[threadIdx.x >> 5];
+    HitRing& R = rings[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        const i64 i = next_row(next);
+        if (i >= n_item) break;
+        const uint2 it = item[i];
+        const int r = (int)it.x;
+        u64 a, b;
+        double psr, cut;
+        row_setup(P, r, a, b, psr, cut);
+        load_lists(S, a, b, P.n_orb);
+        ContractOut out{coeff};
+        QueueEval<ContractOut> q{P, r, a, b, psr, cut, R, out};
+        unsigned long long tests = 0;
+        walk_row<W, true>(P, r, a, b, S, q, tests, (int)(it.y >> 16), (int)(it.y & 0xffffu));
+        q.flush();
+        DDb d = out.acc;
+#pragma unroll
+        for (int o = 16; o; o >>= 1)
+            d.merge(__shfl_xor_sync(0xffffffffu, d.s, o), __shfl_xor_sync(0xffffffffu, d.c, o));
+        if (lane == 0) part[i] = make_double2(d.s, d.c);
+        __syncwarp();
+    }
+}
+
+// Block sum of the threads' compensated sums, valid in thread 0.
+__device__ __forceinline__ DDb block_sum(DDb e) {
+    __shared__ double bs[32], bc[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int o = 16; o; o >>= 1)
+        e.merge(__shfl_xor_sync(0xffffffffu, e.s, o), __shfl_xor_sync(0xffffffffu, e.c, o));
+    if (lane == 0) {
+        bs[w] = e.s;
+        bc[w] = e.c;
+    }
+    __syncthreads();
+    DDb d;
+    if (threadIdx.x == 0)
+        for (int k = 0; k < nw; ++k) d.merge(bs[k], bc[k]);
+    return d;
+}
+
+// sigma of every row from its slices, and the block's share of E.
+__global__ void __launch_bounds__(256)
+k_contract_rows(const u32* order, const i64* off, i64 n, const double* coeff, const double2* part,
+                double* sigma, double2* epart) {
+    DDb e;
+    for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
+         t += (i64)gridDim.x * blockDim.x) {
+        const u32 r = order[t];
+        DDb d;
+        for (i64 k = off[t]; k < off[t + 1]; ++k) d.merge(part[k].x, part[k].y);
+        if (sigma) sigma[r] = d.s + d.c;
+        if (off[t] == off[t + 1]) continue;   // skipped row: sigma 0, no term in E
+        e.add_prod(coeff[r], d.s);
+        e.add_prod(coeff[r], d.c);
+    }
+    e = block_sum(e);
+    if (threadIdx.x == 0) epart[blockIdx.x] = make_double2(e.s, e.c);
+}
+
+__global__ void __launch_bounds__(256) k_contract_final(const double2* epart, int nb, double* out) {
+    DDb e;
+    for (int k = threadIdx.x; k < nb; k += blockDim.x) e.merge(epart[k].x, epart[k].y);
+    e = block_sum(e);
+    if (threadIdx.x == 0) *out = e.s + e.c;
+}
+
 }  // namespace
+
+// E (and sigma, optional) by string groups.  False when the basis lists a
+// determinant twice (its amplitudes then follow the de-duplicated order,
+// which the candidate walk's map holds) or mixes electron counts.  Host synchronisations: the sizes of
+// the indices, the slice count and the result.
+bool contract_strings(dnq_ctx_s* ctx, const u64* V, i64 n, const double* cd, int n_orb,
+                      double single_thr, double cut, double* sigma, cudaStream_t s, double* e) {
+    DBuf<IndexProbe> probe(2, s);
+    DNQ_CUDA(cudaMemsetAsync(probe.p, 0, 2 * sizeof(IndexProbe), s));
+    StrIndex A, B;
+    str_index_begin(A, V, n, 0, n_orb, probe.p, s);
+    str_index_begin(B, V, n, 1, n_orb, probe.p + 1, s);
+    DBuf<u32> mixed(1, s);
+    DNQ_CUDA(cudaMemsetAsync(mixed.p, 0, 4, s));
+    k_mixed_counts<<<gsz(n), 256, 0, s>>>(V, n, mixed.p);
+    DNQ_CHECK_LAUNCH();
+    DBuf<double> diag(n, s);
+    launch_diag(ctx, V, n, diag.p, s);
+    IndexProbe hp[2];
+    u32 hmixed = 0;
+    DNQ_CUDA(cudaMemcpyAsync(hp, probe.p, 2 * sizeof(IndexProbe), cudaMemcpyDeviceToHost, s));
+    DNQ_CUDA(cudaMemcpyAsync(&hmixed, mixed.p, 4, cudaMemcpyDeviceToHost, s));
+    DNQ_CUDA(cudaStreamSynchronize(s));
+    if (hp[0].dup || hmixed) return false;
+    str_index_finish(A, n, hp[0].ngroups, s);
+    str_index_finish(B, n, hp[1].ngroups, s);
+    build_presence_hist(A, B, n, hp[0].hist, s);
+    build_presence_hist(B, A, n, hp[1].hist, s);
+    build_group_cost(A, V, n, 0, n_orb, s);
+    build_group_cost(B, V, n, 1, n_orb, s);
+    DBuf<u32> order;
+    build_row_order(A, B, V, n, n_orb, order, s);
+    VVParams P = make_params(ctx, V, n, n_orb, DNQ_POLICY_STATIC, 0.0, cut, nullptr, diag.p, A, B,
+                             Options{});
+    P.single_thr = single_thr;
+    const bool narrow = n_orb <= 32;
+    int per_sm = 0;
+    if (narrow)
+        DNQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_contract_walk<u32>,
+                                                               kWS * 32, 0));
+    else
+        DNQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_contract_walk<u64>,
+                                                               kWS * 32, 0));
+    const int grid = std::max(1, per_sm) * sm_count(ctx->device);
+    const u32 per = n < 64ll * grid * kWS ? kSliceTests : kSliceTestsMany;
+    DBuf<u32> nsl(n + 1, s);
+    DBuf<i64> off(n + 1, s);
+    k_contract_slices<<<gsz(n + 1), 256, 0, s>>>(P, order.p, cd, per, nsl.p);
+    DNQ_CHECK_LAUNCH();
+    prim::scan<u32, i64, false>(nsl.p, off.p, n + 1, s);
+    i64 items = 0;
+    DNQ_CUDA(cudaMemcpyAsync(&items, off.p + n, 8, cudaMemcpyDeviceToHost, s));
+    DNQ_CUDA(cudaStreamSynchronize(s));
+    require(items < (i64)0x7fffffffll - 65536, DNQ_ERR_OVERFLOW, "too many rows to contract");
+    DBuf<uint2> item(items, s);
+    DBuf<double2> part(items, s);
+    DBuf<int> next(1, s);
+    DNQ_CUDA(cudaMemsetAsync(next.p, 0, 4, s));
+    k_contract_items<<<gsz(n), 256, 0, s>>>(order.p, nsl.p, off.p, n, item.p);
+    DNQ_CHECK_LAUNCH();
+    if (narrow)
+        k_contract_walk<u32><<<grid, kWS * 32, 0, s>>>(P, cd, item.p, items, next.p, part.p);
+    else
+        k_contract_walk<u64><<<grid, kWS * 32, 0, s>>>(P, cd, item.p, items, next.p, part.p);
+    DNQ_CHECK_LAUNCH();
+    const int nb = (int)std::min<i64>((n + 255) / 256, 2 * sm_count(ctx->device));
+    DBuf<double2> epart(nb, s);
+    DBuf<double> out(1, s);
+    k_contract_rows<<<nb, 256, 0, s>>>(order.p, off.p, n, cd, part.p, sigma, epart.p);
+    DNQ_CHECK_LAUNCH();
+    k_contract_final<<<1, 256, 0, s>>>(epart.p, nb, out.p);
+    DNQ_CHECK_LAUNCH();
+    DNQ_CUDA(cudaMemcpyAsync(e, out.p, 8, cudaMemcpyDeviceToHost, s));
+    DNQ_CUDA(cudaStreamSynchronize(s));
+    return true;
+}
+
 }  // namespace dnq
 
 struct dnq_batch_s {

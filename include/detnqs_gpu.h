@@ -158,7 +158,9 @@ int dnq_ham_destroy(dnq_ham_t h);
  * code path with small inputs):
  *   DNQ_OPT_FORCE_WALK  1: route V->V-only builds through the per-row
  *                          candidate walk instead of the string-group
- *                          matcher (both give identical blocks);
+ *                          matcher (both give identical blocks), and
+ *                          matrix-free contractions likewise (read when
+ *                          the call starts);
  *   DNQ_OPT_ARENA_CHUNK n: entries per warp chunk of the single-pass V->V
  *                          build (0 = default: 8192, and 16384 for
  *                          single builds of at least 64 rows per
