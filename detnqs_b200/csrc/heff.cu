@@ -403,29 +403,297 @@ __global__ void k_long_terms(const u32* vpcol, const double* vpval, const i64* p
     }
 }
 
-// FP64: the terms summed in k order by one thread (the order of the
-// reference's accumulation, so the result is bit-identical).  The block
-// stages chunks of the terms in shared memory so the summing thread reads
-// them at shared-memory latency.
-constexpr int kSumChunk = 4096;
-__global__ void __launch_bounds__(1024) k_long_sum64(const double* term, i64 n, double* out) {
-    __shared__ double sh[kSumChunk];
-    double acc = 0.0;
-    for (i64 c0 = 0; c0 < n; c0 += kSumChunk) {
-        const int m = (int)min((i64)kSumChunk, n - c0);
-        for (int t = threadIdx.x; t < m; t += blockDim.x) sh[t] = term[c0 + t];
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int t = 0;
-            for (; t + 8 <= m; t += 8) {
+// FP64: acc + term[0] + term[1] + ... with the rounding of that order of
+// additions (the reference's), bit for bit, but not one at a time.  While the
+// sum stays in one binade its spacing u is fixed: acc = S u with S an integer
+// in [2^52, 2^53), and adding a term x u rounds to (S + rint(x)) u unless x
+// lies half way between integers (then the parity of S decides).  So a tile of
+// terms becomes integers, their prefix sums are exact in 64 bits, and the tile
+// is taken up to the first place where a partial sum leaves the binade or a
+// term is such a tie.  Thread 0 adds a few terms in the plain way from there
+// and the tile goes on in the new binade.  A sum of n terms of one sign passes
+// about log2(n) binades; sums that turn or start small take longer plain runs
+// (the run doubles while the parallel step gets nowhere), so the worst input
+// costs about the plain loop's time twice.
+//
+// The plain loop is bound by the latency of one FP64 addition: 18.5 ms for
+// the 3.75e6 terms of a Hartree-Fock row of 100 orbitals.  One block that
+// takes tile after tile this way still spends 2.7 ms on conversions and
+// barriers, so the tiles are converted by the whole grid: the plain sums of
+// the tiles (k_sum_tiles) give the binade each is likely to start in, every
+// block turns its tile into integers of that binade and keeps their total and
+// the extremes of their prefix sums (k_sum_units), and one block walks the
+// tiles with a few integer operations each (k_long_sum64), going through a
+// tile's terms only where the guess or the binade does not hold.
+constexpr int kSumThreads = 256;
+constexpr int kSumItems = 8;
+constexpr int kSumTile = kSumThreads * kSumItems;
+
+struct SumUnit {
+    long long total;      // of the tile's integers
+    long long lo, hi;     // extremes of their inclusive prefix sums
+    int exp;              // binade they were made for; kNoBinade: not usable
+    int neg;              // sign of the sum they were made for
+};
+constexpr int kNoBinade = 0x7fffffff;
+
+__device__ __forceinline__ bool sum_in_range(double mag) {
+    return mag >= 0x1p-900 && mag < 0x1p+900;   // false for NaN
+}
+__device__ __forceinline__ int sum_exp(double mag) {
+    return (int)((__double_as_longlong(mag) >> 52) & 0x7ff) - 1023;
+}
+__device__ __forceinline__ double pow2(int e) {
+    return __longlong_as_double((long long)(1023 + e) << 52);
+}
+
+// Sum of each tile, in any order.
+__global__ void __launch_bounds__(kSumThreads) k_sum_tiles(const double* term, i64 n,
+                                                           double* tsum) {
+    __shared__ double ws[kSumThreads / 32];
+    const i64 c0 = (i64)blockIdx.x * kSumTile;
+    double a = 0.0;
 #pragma unroll
-                for (int q = 0; q < 8; ++q) acc = __dadd_rn(acc, sh[t + q]);
+    for (int i = 0; i < kSumItems; ++i) {
+        const i64 t = c0 + (i64)i * kSumThreads + threadIdx.x;
+        if (t < n) a += term[t];
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = a;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < kSumThreads / 32; ++k) a += ws[k];
+        tsum[blockIdx.x] = a;
+    }
+}
+
+// The integers of a thread's kSumItems terms for the binade of `scale` (a
+// signed power of two); bit i of the result: term i may not be taken so.
+__device__ __forceinline__ u32 sum_integers(const double* x, double scale, long long* q) {
+    u32 odd = 0;
+#pragma unroll
+    for (int i = 0; i < kSumItems; ++i) {
+        const double y = x[i] * scale;
+        const double r = rint(y);
+        const bool ok = fabs(y) < 0x1p+53 && fabs(y - r) != 0.5;   // false for NaN
+        q[i] = ok ? (long long)r : 0ll;
+        odd |= (ok ? 0u : 1u) << i;
+    }
+    return odd;
+}
+
+// The block's terms in thread order: thread t gets x[0..kSumItems) = term
+// t * kSumItems + i of the tile (0 past the end), loaded coalesced.
+__device__ __forceinline__ void sum_load(const double* term, i64 n, i64 c0, double* sh,
+                                         double* x) {
+#pragma unroll
+    for (int i = 0; i < kSumItems; ++i) {
+        const i64 t = c0 + (i64)i * kSumThreads + threadIdx.x;
+        sh[i * kSumThreads + threadIdx.x] = t < n ? term[t] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kSumItems; ++i) x[i] = sh[threadIdx.x * kSumItems + i];
+}
+
+// Exclusive prefix over the block of each thread's value (modulo 2^64), and
+// the block's total.
+__device__ __forceinline__ long long sum_prefix(long long v, long long* ws, long long* all) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned long long incl = (unsigned long long)v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    __syncthreads();   // ws is free
+    if (lane == 31) ws[w] = (long long)incl;
+    __syncthreads();
+    unsigned long long before = 0, tot = 0;
+#pragma unroll
+    for (int k = 0; k < kSumThreads / 32; ++k) {
+        if (k < w) before += (unsigned long long)ws[k];
+        tot += (unsigned long long)ws[k];
+    }
+    *all = (long long)tot;
+    return (long long)(before + incl - (unsigned long long)v);
+}
+
+__global__ void __launch_bounds__(kSumThreads) k_sum_units(const double* term, i64 n,
+                                                           const double* tsum, SumUnit* unit) {
+    __shared__ double sh[kSumTile];
+    __shared__ long long ws[kSumThreads / 32];
+    __shared__ double est_sh[kSumThreads / 32];
+    __shared__ long long lo_sh, hi_sh;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // the sum in front of this tile, roughly
+    double est = 0.0;
+    for (int k = threadIdx.x; k < (int)blockIdx.x; k += kSumThreads) est += tsum[k];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) est += __shfl_xor_sync(0xffffffffu, est, o);
+    if (lane == 0) est_sh[w] = est;
+    if (threadIdx.x == 0) {
+        lo_sh = 0x7fffffffffffffffll;
+        hi_sh = -0x7fffffffffffffffll;
+    }
+    double x[kSumItems];
+    sum_load(term, n, (i64)blockIdx.x * kSumTile, sh, x);
+    est = 0.0;
+    for (int k = 0; k < kSumThreads / 32; ++k) est += est_sh[k];
+    const double mag = fabs(est);
+    const bool good = sum_in_range(mag);
+    const int e = good ? sum_exp(mag) : 0;
+    long long q[kSumItems], tot = 0;
+    const u32 odd = sum_integers(x, copysign(pow2(52 - e), est), q);
+#pragma unroll
+    for (int i = 0; i < kSumItems; ++i) tot += q[i];   // |q| <= 2^53: no overflow in a thread
+    long long all = 0;
+    long long v = sum_prefix(tot, ws, &all);
+    // 2048 integers of up to 2^53 may overflow their sum: such terms are as
+    // large as the sum itself and end the binade, so the tile is not usable
+    bool bad = odd != 0;
+    long long lo = 0x7fffffffffffffffll, hi = -0x7fffffffffffffffll;
+#pragma unroll
+    for (int i = 0; i < kSumItems; ++i) {
+        bad = bad || q[i] > (1ll << 50) || q[i] < -(1ll << 50);   // 2^11 of them stay below 2^61
+        v += q[i];
+        lo = min(lo, v);
+        hi = max(hi, v);
+    }
+    atomicMin(&lo_sh, lo);
+    atomicMax(&hi_sh, hi);
+    const bool any = __syncthreads_or(bad);
+    if (threadIdx.x == 0)
+        unit[blockIdx.x] = SumUnit{all, lo_sh, hi_sh, good && !any ? e : kNoBinade, est < 0.0};
+}
+
+// acc plus the m terms of one tile, through the block: integer prefix sums
+// up to the first place that may not be taken, a plain run from there, and
+// again.
+__device__ double sum_tile(double acc, const double* term, i64 n, i64 c0, int m, double* sh,
+                           long long* ws, int* s_stop, double* s_acc) {
+    const int tid = threadIdx.x, t0 = tid * kSumItems;
+    double x[kSumItems];
+    __syncthreads();
+    sum_load(term, n, c0, sh, x);
+    int pos = 0, run = 16;
+    while (pos < m) {   // pos, run and acc are block-uniform
+        int stop = pos;
+        const double mag = fabs(acc);
+        if (m - pos >= 64 && sum_in_range(mag)) {
+            const int e = sum_exp(mag);
+            double y[kSumItems];
+#pragma unroll
+            for (int i = 0; i < kSumItems; ++i) y[i] = t0 + i >= pos && t0 + i < m ? x[i] : 0.0;
+            long long q[kSumItems], tot = 0, all = 0;
+            const u32 odd = sum_integers(y, copysign(pow2(52 - e), acc), q);
+#pragma unroll
+            for (int i = 0; i < kSumItems; ++i) tot += q[i];
+            if (tid == 0) *s_stop = m;
+            // exact up to the first prefix out of range: those before it are
+            // below 2^53, and so is a term
+            const long long S0 = (long long)(mag * pow2(52 - e));
+            const long long before =
+                (long long)((unsigned long long)S0 + (unsigned long long)sum_prefix(tot, ws, &all));
+            unsigned long long v = (unsigned long long)before;
+            int bad = m;
+#pragma unroll
+            for (int i = 0; i < kSumItems; ++i) {
+                v += (unsigned long long)q[i];
+                const bool in = (long long)v > (1ll << 52) && (long long)v < (1ll << 53);
+                if (bad == m && t0 + i >= pos && t0 + i < m && (!in || ((odd >> i) & 1u)))
+                    bad = t0 + i;
             }
-            for (; t < m; ++t) acc = __dadd_rn(acc, sh[t]);
+            if (bad < m) atomicMin(s_stop, bad);
+            __syncthreads();
+            stop = *s_stop;
+            // the thread that holds the last place taken writes the sum there
+            const int last = stop - 1;
+            if (stop > pos && last / kSumItems == tid) {
+                v = (unsigned long long)before;
+#pragma unroll
+                for (int k = 0; k < kSumItems; ++k)
+                    if (k <= last % kSumItems) v += (unsigned long long)q[k];
+                *s_acc = copysign((double)(long long)v * pow2(e - 52), acc);
+            }
+            __syncthreads();
+            if (stop > pos) acc = *s_acc;
+            run = stop - pos >= 256 ? 16 : min(2 * run, kSumTile);
+        } else {
+            run = min(2 * run, kSumTile);
         }
+        if (stop < m) {   // a plain run from the stop
+            const int end = m - stop < 64 ? m : min(m, stop + run);
+            __syncthreads();
+            if (tid == 0) {
+                double a = acc;
+                for (int t = stop; t < end; ++t) a = __dadd_rn(a, sh[t]);
+                *s_acc = a;
+            }
+            __syncthreads();
+            acc = *s_acc;
+            stop = end;
+        }
+        pos = stop;
         __syncthreads();
     }
+    return acc;
+}
+
+__global__ void __launch_bounds__(kSumThreads) k_long_sum64(const double* term, i64 n,
+                                                            const SumUnit* unit, int nu,
+                                                            double* out) {
+    __shared__ SumUnit us[kSumThreads];
+    __shared__ double sh[kSumTile];
+    __shared__ long long ws[kSumThreads / 32];
+    __shared__ int s_stop, s_next;
+    __shared__ double s_acc;
+    double acc = 0.0;   // the same in every thread
+    for (int u0 = 0; u0 < nu; u0 += kSumThreads) {
+        const int nk = min(kSumThreads, nu - u0);
+        __syncthreads();
+        if ((int)threadIdx.x < nk) us[threadIdx.x] = unit[u0 + threadIdx.x];
+        __syncthreads();
+        int k = 0;
+        while (k < nk) {
+            if (threadIdx.x == 0) {   // whole tiles while their binade holds
+                double a = acc;
+                for (; k < nk; ++k) {
+                    const SumUnit t = us[k];
+                    const double mag = fabs(a);
+                    if (!sum_in_range(mag) || t.exp != sum_exp(mag) || t.neg != (a < 0.0)) break;
+                    const long long S = (long long)(mag * pow2(52 - t.exp));
+                    if (!(S + t.lo > (1ll << 52) && S + t.hi < (1ll << 53))) break;
+                    a = copysign((double)(S + t.total) * pow2(t.exp - 52), a);
+                }
+                s_acc = a;
+                s_next = k;
+            }
+            __syncthreads();
+            acc = s_acc;
+            k = s_next;
+            if (k < nk) {
+                const i64 c0 = (i64)(u0 + k) * kSumTile;
+                acc = sum_tile(acc, term, n, c0, (int)min((i64)kSumTile, n - c0), sh, ws, &s_stop,
+                               &s_acc);
+                ++k;
+            }
+            __syncthreads();
+        }
+    }
     if (threadIdx.x == 0) *out = acc;
+}
+
+void long_sum64(const double* term, i64 n, double* out, cudaStream_t s) {
+    const i64 nu = (n + kSumTile - 1) / kSumTile;
+    DBuf<double> tsum(nu, s);
+    DBuf<SumUnit> unit(nu, s);
+    k_sum_tiles<<<(unsigned)nu, kSumThreads, 0, s>>>(term, n, tsum.p);
+    DNQ_CHECK_LAUNCH();
+    k_sum_units<<<(unsigned)nu, kSumThreads, 0, s>>>(term, n, tsum.p, unit.p);
+    DNQ_CHECK_LAUNCH();
+    k_long_sum64<<<1, kSumThreads, 0, s>>>(term, n, unit.p, (int)nu, out);
 }
 
 // FP32: float-float sums over a fixed tree: kSum32Blocks x 256 threads each
@@ -745,7 +1013,7 @@ void ham_eff_csr(const Csr& VV, const Csr& VP, i64 nv, i64 np, const double* hpp
                 DNQ_CHECK_LAUNCH();
                 k_long_merge32<<<1, 32, 0, s>>>(part.p, ldiag2.p + q);
             } else {
-                k_long_sum64<<<1, 1024, 0, s>>>(term.p, m, ldiag.p + q);
+                long_sum64(term.p, m, ldiag.p + q, s);
             }
             DNQ_CHECK_LAUNCH();
             // kept k's whose column holds other rows, in order
