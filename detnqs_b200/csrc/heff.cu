@@ -22,6 +22,7 @@
 //      order from the bitmap.
 
 #include <memory>
+#include <type_traits>
 #include <vector>
 
 #include "ham.cuh"
@@ -157,19 +158,25 @@ struct HeffParams {
 
 // F32 = false: acc holds FP64 sums.  F32 = true: during the scatter acc
 // holds (sum, err) float pairs, folded to FP64 before H_VV is added.
+//
+// Bound: latency.  The sums into one element follow k, so a warp takes its
+// columns one after the other, and the accumulators leave room for few warps
+// (12 per SM at 2,241 rows).  The columns' entries are therefore read kHeffU
+// steps of 32 ahead of their additions, across column ends, a batch's metadata
+// one batch ahead, and a touched bit is set atomically only where it is not
+// set yet.
+// Measured on 2,241 rows, 4.35e6 H_VP entries, 147,420 columns: 4.66 ms
+// with one column at a time in flight and a bitmap of touched elements, 1.60 now.
+constexpr int kHeffU = 8;
 template <bool F32, bool SMEM>
 __global__ void __launch_bounds__(kHW * 32) k_heff(HeffParams P) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const i64 gw = (i64)blockIdx.x * kHW + w;
-    u32* bits;
+    u32* bits = nullptr;   // touched columns; in shared memory the row is swept whole
     double* acc;
     if (SMEM) {
-        const size_t per = (((size_t)P.words * 4 + 15) & ~(size_t)15) + (size_t)P.nv * 8;
-        unsigned char* base = smem + per * w;
-        bits = (u32*)base;
-        acc = (double*)(base + (((size_t)P.words * 4 + 15) & ~(size_t)15));
-        for (int t = lane; t < P.words; t += 32) bits[t] = 0u;
+        acc = (double*)smem + (size_t)P.nv * w;
         for (i64 t = lane; t < P.nv; t += 32) acc[t] = 0.0;
         __syncwarp();
     } else {
@@ -177,6 +184,11 @@ __global__ void __launch_bounds__(kHW * 32) k_heff(HeffParams P) {
         acc = P.gacc + gw * P.nv;
     }
     float2* acc2 = reinterpret_cast<float2*>(acc);
+    using V = typename std::conditional<F32, float, double>::type;   // stored H_PV values
+    using S1 = V;                                                    // a * D^-1
+    const V* pv;
+    if constexpr (F32) pv = P.pvval32;
+    else pv = P.pvval;
     for (;;) {
         int i = 0;
         if (lane == 0) i = atomicAdd(P.next_row, 1);
@@ -194,7 +206,7 @@ __global__ void __launch_bounds__(kHW * 32) k_heff(HeffParams P) {
         if (lid >= 0) {   // precomputed sums of a long row (same order, same values)
             for (i64 x = P.long_off[lid] + lane; x < P.long_off[lid + 1]; x += 32) {
                 const u32 j = P.long_j[x];
-                atomicOr(&bits[j >> 5], 1u << (j & 31));
+                if constexpr (!SMEM) atomicOr(&bits[j >> 5], 1u << (j & 31));
                 if (F32) acc2[j] = P.long_v2[x];
                 else acc[j] = P.long_v[x];
             }
@@ -202,90 +214,133 @@ __global__ void __launch_bounds__(kHW * 32) k_heff(HeffParams P) {
         }
         const i64 t_base = P.vprp[i];
         const i64 n_items = lid >= 0 ? 0 : P.vprp[i + 1] - t_base;
-        for (i64 x0 = 0; x0 < n_items; x0 += 32) {
-            const i64 xl = x0 + lane;
-            const bool inr = xl < n_items;
-            const i64 tl = inr ? t_base + xl : 0;
-            u32 kl = 0;
-            bool sk = true;
-            double al = 0.0, sl = 0.0;
-            i64 q0l = 0, q1l = 0, qdl = -1;
-            if (inr) {
-                kl = P.vpcol[tl];
-                sk = P.skip[kl] != 0;
-                sl = P.dinv[kl];
-                al = F32 ? (double)P.vpval32[tl] : P.vpval[tl];
-                q0l = P.pvrp[kl];
-                q1l = P.pvrp[kl + 1];
-                i64 lo = q0l, hi = q1l;   // position of row i in column k
-                while (lo < hi) {
-                    const i64 mid = (lo + hi) >> 1;
-                    if (P.pvcol[mid] < (u32)i) lo = mid + 1; else hi = mid;
-                }
-                qdl = lo;
+        // A batch is 32 k's, one per lane; the metadata of the next batch and
+        // the k's of the one after it are read while a batch is worked on.
+        // H_PV[k, i] is the stored value H_VP[i, k] (the transpose copies it).
+        struct Meta {
+            bool sk;
+            double a, s;
+            i64 q0, q1;
+        };
+        auto k_of = [&](i64 x0) {
+            return x0 + lane < n_items ? P.vpcol[t_base + x0 + lane] : 0xffffffffu;
+        };
+        auto meta_of = [&](i64 x0, u32 k) {
+            Meta m{true, 0.0, 0.0, 0, 0};
+            if (x0 + lane < n_items) {
+                m.sk = P.skip[k] != 0;
+                m.s = P.dinv[k];
+                m.a = F32 ? (double)P.vpval32[t_base + x0 + lane] : P.vpval[t_base + x0 + lane];
+                m.q0 = P.pvrp[k];
+                m.q1 = P.pvrp[k + 1];
             }
-            const double bdl = (inr && !sk) ? (F32 ? (double)P.pvval32[qdl] : P.pvval[qdl]) : 0.0;
-            const int cnt = (int)min((i64)32, n_items - x0);
-            for (int u = 0; u < cnt; ++u) {
-                if (__shfl_sync(0xffffffffu, (int)sk, u)) continue;
-                const double s = __shfl_sync(0xffffffffu, sl, u);
-                const double a = __shfl_sync(0xffffffffu, al, u);
-                const i64 q0 = __shfl_sync(0xffffffffu, q0l, u);
-                const i64 q1 = __shfl_sync(0xffffffffu, q1l, u);
-                const i64 qd = __shfl_sync(0xffffffffu, qdl, u);
-                const double bd = __shfl_sync(0xffffffffu, bdl, u);
-                const bool need = !(a == 0.0 || s == 0.0);
-                if (!F32) {
-                    const double as = __dmul_rn(a, s);
-                    if (lane == 0 && lid < 0) {
-                        dtouch = true;
-                        if (need) dacc = __dadd_rn(dacc, __dmul_rn(as, bd));
-                    }
-                    if (q1 - q0 > 1) {
-                        for (i64 q = q0 + lane; q < q1; q += 32) {
-                            if (q == qd) continue;
-                            const u32 j = P.pvcol[q];
-                            atomicOr(&bits[j >> 5], 1u << (j & 31));
-                            if (need) acc[j] = __dadd_rn(acc[j], __dmul_rn(as, P.pvval[q]));
-                        }
-                    }
+            return m;
+        };
+        u32 k_next = k_of(0);
+        Meta next = meta_of(0, k_next);
+        k_next = k_of(32);
+        for (i64 x0 = 0; x0 < n_items; x0 += 32) {
+            const Meta me = next;
+            next = meta_of(x0 + 32, k_next);
+            k_next = k_of(x0 + 64);
+            const unsigned kept = __ballot_sync(0xffffffffu, !me.sk);
+            if (kept == 0) continue;
+            const bool need_l = !(me.a == 0.0 || me.s == 0.0);
+            const unsigned needed = __ballot_sync(0xffffffffu, need_l && !me.sk);
+            const double as_l = __dmul_rn(me.a, me.s);
+            // a * D^-1 as a float pair hi + lo (F32: the FP64 shift keeps its
+            // precision; only stored values are FP32)
+            const float ash_l = (float)as_l;
+            const float asl_l = (float)(as_l - (double)ash_l);
+            // Float-float accumulation: TwoProduct and TwoSum errors go to the
+            // error word, renormalised after each add (FastTwoSum; Dekker 1971).
+            auto add = [](float& hi, float& lo, float as, float as_lo, float b) {
+                const float p = __fmul_rn(as, b);
+                const float pe = fmaf(as, b, -p) + __fmul_rn(as_lo, b);
+                float s2, e;
+                f_two_sum(hi, p, s2, e);
+                const float c = __fadd_rn(lo, __fadd_rn(e, pe));
+                hi = __fadd_rn(s2, c);
+                lo = __fsub_rn(c, __fsub_rn(hi, s2));
+            };
+            // the diagonal element: one term per kept k, in order (every lane
+            // keeps the same sum)
+            dtouch = true;
+            const double dt_l = __dmul_rn(as_l, me.a);
+            for (unsigned m = needed; m; m &= m - 1) {
+                const int u = __ffs(m) - 1;
+                if constexpr (!F32) {
+                    dacc = __dadd_rn(dacc, __shfl_sync(0xffffffffu, dt_l, u));
                 } else {
-                    // a * D^-1 in FP64, carried as a float pair hi + lo (the
-                    // FP64 shift keeps its precision; only stored values are
-                    // FP32)
-                    const double asd = __dmul_rn(a, s);
-                    const float as = (float)asd;
-                    const float as_lo = (float)(asd - (double)as);
-                    auto add = [&](float& hi, float& lo, float b) {
-                        // float-float accumulation: TwoProduct and TwoSum errors
-                        // go to the error word, renormalised after each add
-                        // (FastTwoSum; Dekker 1971)
-                        const float p = __fmul_rn(as, b);
-                        const float pe = fmaf(as, b, -p) + __fmul_rn(as_lo, b);
-                        float s2, e;
-                        f_two_sum(hi, p, s2, e);
-                        const float c = __fadd_rn(lo, __fadd_rn(e, pe));
-                        hi = __fadd_rn(s2, c);
-                        lo = __fsub_rn(c, __fsub_rn(hi, s2));
-                    };
-                    if (lane == 0 && lid < 0) {
-                        dtouch = true;
-                        if (need) add(dhi, dlo, (float)bd);
+                    add(dhi, dlo, __shfl_sync(0xffffffffu, ash_l, u),
+                        __shfl_sync(0xffffffffu, asl_l, u),
+                        (float)__shfl_sync(0xffffffffu, me.a, u));
+                }
+            }
+            // the other elements: steps of 32 entries of one column, columns in
+            // order, kHeffU steps in flight
+            unsigned cols = __ballot_sync(0xffffffffu, !me.sk && me.q1 - me.q0 > 1);
+            i64 q = 0, qe = 0;
+            int u = 0;
+            bool some[kHeffU];   // there is such a step (they come in order)
+            u32 js[kHeffU];      // this lane's element, ~0: none
+            V bs[kHeffU];
+            S1 as[kHeffU];       // the column's a * D^-1
+            float as_lo[kHeffU];
+            bool need[kHeffU];
+            auto fetch = [&](int v) {
+                some[v] = false;
+                if (q >= qe) {
+                    if (!cols) return;
+                    u = __ffs(cols) - 1;
+                    cols &= cols - 1;
+                    q = __shfl_sync(0xffffffffu, me.q0, u);
+                    qe = __shfl_sync(0xffffffffu, me.q1, u);
+                }
+                some[v] = true;
+                js[v] = 0xffffffffu;
+                if (q + lane < qe) {
+                    js[v] = P.pvcol[q + lane];
+                    bs[v] = pv[q + lane];
+                }
+                need[v] = (needed >> u) & 1u;
+                if constexpr (!F32) {
+                    as[v] = __shfl_sync(0xffffffffu, as_l, u);
+                } else {
+                    as[v] = __shfl_sync(0xffffffffu, ash_l, u);
+                    as_lo[v] = __shfl_sync(0xffffffffu, asl_l, u);
+                }
+                q += 32;
+            };
+#pragma unroll
+            for (int v = 0; v < kHeffU; ++v) fetch(v);
+            for (bool more = some[0]; more;) {
+#pragma unroll
+                for (int v = 0; v < kHeffU; ++v) {
+                    if (!some[v]) {
+                        more = false;
+                        break;
                     }
-                    if (q1 - q0 > 1) {
-                        for (i64 q = q0 + lane; q < q1; q += 32) {
-                            if (q == qd) continue;
-                            const u32 j = P.pvcol[q];
-                            atomicOr(&bits[j >> 5], 1u << (j & 31));
-                            if (need) {
-                                float2 cur = acc2[j];
-                                add(cur.x, cur.y, P.pvval32[q]);
-                                acc2[j] = cur;
-                            }
+                    const u32 j = js[v];
+                    const bool on = j != 0xffffffffu && j != (u32)i;
+                    if constexpr (!SMEM) {
+                        if (on) {   // most bits are set already
+                            const u32 bit = 1u << (j & 31);
+                            if (!(bits[j >> 5] & bit)) atomicOr(&bits[j >> 5], bit);
                         }
                     }
+                    if (on && need[v]) {
+                        if constexpr (!F32) {
+                            acc[j] = __dadd_rn(acc[j], __dmul_rn(as[v], bs[v]));
+                        } else {
+                            float2 cur = acc2[j];
+                            add(cur.x, cur.y, as[v], as_lo[v], bs[v]);
+                            acc2[j] = cur;
+                        }
+                    }
+                    fetch(v);
+                    __syncwarp();   // another lane may hold this j in the next step
                 }
-                __syncwarp();
             }
         }
         if (lid >= 0 && lane == 0) {
@@ -296,11 +351,47 @@ __global__ void __launch_bounds__(kHW * 32) k_heff(HeffParams P) {
             dlo = d2.y;
         }
         if (lane == 0 && dtouch) {
-            atomicOr(&bits[i >> 5], 1u << (i & 31));
+            if constexpr (!SMEM) atomicOr(&bits[i >> 5], 1u << (i & 31));
             if (F32) acc2[i] = make_float2(dhi, dlo);
             else acc[i] = dacc;
         }
         __syncwarp();
+        i64 wpos = P.capoff[i];
+        u32 written = 0;
+        if constexpr (SMEM) {
+            // fold the FP32 pairs, add H_VV row i (csr_add: vv + add; an
+            // untouched element is 0, and adds nothing), then sweep the row in
+            // column order: keep |v| > 1e-15 and clear
+            if (F32) {
+                for (i64 j = lane; j < P.nv; j += 32) {
+                    const float2 pr = acc2[j];
+                    acc[j] = (double)pr.x + (double)pr.y;
+                }
+                __syncwarp();
+            }
+            for (i64 t = P.vvrp[i] + lane; t < P.vvrp[i + 1]; t += 32) {
+                const u32 j = P.vvcol[t];
+                acc[j] = __dadd_rn(P.vvval[t], acc[j]);
+            }
+            __syncwarp();
+            for (i64 j0 = 0; j0 < P.nv; j0 += 32) {
+                const i64 j = j0 + lane;
+                const double v = j < P.nv ? acc[j] : 0.0;
+                if (j < P.nv) acc[j] = 0.0;
+                const bool keep = fabs(v) > 1e-15;
+                const unsigned m = __ballot_sync(0xffffffffu, keep);
+                if (keep) {
+                    const i64 at = wpos + __popc(m & lanemask_lt());
+                    P.tcol[at] = (u32)j;
+                    P.tval[at] = v;
+                }
+                wpos += __popc(m);
+                written += __popc(m);
+            }
+            if (lane == 0) P.rowcnt[i] = written;
+            __syncwarp();
+            continue;
+        }
         if (F32) {   // fold (sum, err) pairs to FP64
             for (int wd = lane; wd < P.words; wd += 32)
                 for (u32 m = bits[wd]; m; m &= m - 1) {
@@ -320,8 +411,6 @@ __global__ void __launch_bounds__(kHW * 32) k_heff(HeffParams P) {
         }
         __syncwarp();
         // ---- compact in column order, keep |v| > 1e-15, clear the slab
-        i64 wpos = P.capoff[i];
-        u32 written = 0;
         for (int w0 = 0; w0 < P.words; w0 += 32) {
             const int wd = w0 + lane;
             const u32 word = wd < P.words ? bits[wd] : 0u;
@@ -367,6 +456,27 @@ __global__ void k_compact(const i64* capoff, const u32* tcol, const double* tval
             col[dst + t] = tcol[src + t];
             val[dst + t] = tval[src + t];
         }
+    }
+}
+
+// Diagonal entry of every row (0 where the row keeps none), columns in any
+// order; warp per row.
+__global__ void k_diag_entry(const i64* rp, const u32* col, const double* val, i64 n, double* out) {
+    const int lane = threadIdx.x & 31;
+    const i64 gw = (blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5;
+    const i64 nw = (gridDim.x * (i64)blockDim.x) >> 5;
+    for (i64 r = gw; r < n; r += nw) {
+        double d = 0.0;
+        for (i64 k0 = rp[r]; k0 < rp[r + 1]; k0 += 32) {
+            const i64 k = k0 + lane;
+            const bool on = k < rp[r + 1] && (i64)col[k] == r;
+            const unsigned m = __ballot_sync(0xffffffffu, on);
+            if (m) {
+                d = __shfl_sync(0xffffffffu, on ? val[k] : 0.0, __ffs(m) - 1);
+                break;
+            }
+        }
+        if (lane == 0) out[r] = d;
     }
 }
 
@@ -902,6 +1012,16 @@ void coo_to_csr_dev(const u32* r, const u32* c, const double* v, i64 n, i64 nr, 
     scan_excl(rowcnt.p, out.rowptr.p, nr + 1, s);
 }
 
+// The stored diagonal of H's V block for dnq_ham_copy_diag.
+void keep_diagonal(dnq_ham_s* H, cudaStream_t s) {
+    const i64 n = H->vv.nr;
+    if (n == 0) return;
+    H->diag.alloc(n, s);
+    k_diag_entry<<<gs(32 * n), 256, 0, s>>>(H->vv.rowptr.p, H->vv.col.p, H->vv.val.p, n,
+                                            H->diag.p);
+    DNQ_CHECK_LAUNCH();
+}
+
 }  // namespace
 
 // Core of the downfolding on canonical CSR blocks (VV: nv x nv, VP: nv x np).
@@ -1101,7 +1221,7 @@ void ham_eff_csr(const Csr& VV, const Csr& VP, i64 nv, i64 np, const double* hpp
         P.long_diag2 = ldiag2.p;
         P.long_touch = ltouch.p;
     }
-    const size_t per_warp = (((size_t)P.words * 4 + 15) & ~(size_t)15) + (size_t)nv * 8;
+    const size_t per_warp = (size_t)nv * 8;
     const bool smem = per_warp * kHW <= 200 * 1024;
     const int sms = sm_count(device);
     DBuf<double> gacc;
@@ -1142,6 +1262,7 @@ void ham_eff_csr(const Csr& VV, const Csr& VP, i64 nv, i64 np, const double* hpp
     k_compact<<<sms * 4, 256, 0, s>>>(capoff.p, tcol.p, tval.p, H->vv.rowptr.p, nv, H->vv.col.p,
                                       H->vv.val.p);
     DNQ_CHECK_LAUNCH();
+    keep_diagonal(H, s);
     DNQ_CUDA(cudaStreamSynchronize(s));
 }
 
@@ -1156,6 +1277,7 @@ void ham_eff(const u32* vvr, const u32* vvc, const double* vvv, i64 vvn, i64 nv,
     coo_to_csr_dev(vvr, vvc, vvv, vvn, nv, nv, VV, s);
     if (np == 0) {   // ham_eff.cpp:72-77: H_VV canonicalised
         H->vv = std::move(VV);
+        keep_diagonal(H, s);
         DNQ_CUDA(cudaStreamSynchronize(s));
         return;
     }
@@ -1200,6 +1322,7 @@ int dnq_ham_eff_from(dnq_ham_t proxy, const double* h_pp, double e_ref, int reg_
         H->stream = s;
         H->n_v = proxy->n_v;
         H->vv = std::move(copy);
+        keep_diagonal(H.get(), s);
         DNQ_CUDA(cudaStreamSynchronize(s));
     } else {
         DIn<double> hpp(h_pp, proxy->n_p, s);

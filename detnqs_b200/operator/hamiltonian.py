@@ -178,7 +178,7 @@ def build_effective_hamiltonian(
                                    None, C.byref(h)))
     H = DeviceHamiltonian(h.value)
     return VVHamiltonian(ham_vv=DeviceBlock(H, 0),
-                         diagonals=DiagonalInfo(V=np.asarray(H.to_scipy(0).diagonal()),
+                         diagonals=DiagonalInfo(V=H.diagonal(),
                                                 P=np.zeros((0,), np.float64)))
 
 
