@@ -10,21 +10,33 @@
 //   * the row sort keeps a block per row in shared memory (bitonic network)
 //     and sends only rows longer than a block holds through the global sort.
 //
-// Radix sort: per pass of 8 bits, k_radix_hist counts the digits of each
-// tile of 2048 keys (warp-aggregated with __match_any_sync), the digit-major
-// table of counts is prefix-summed, and k_radix_scatter ranks every key
-// inside its tile -- each warp walks its 256 keys in 8 rounds of 32 in input
-// order, a key's rank is the count of its digit in earlier rounds plus its
-// lanes before it in the round, and warps are offset per digit -- and writes
-// it at (digits below + same digit in earlier tiles + rank).  Equal digits
-// keep their input order, so the passes compose into a stable sort.
+// Radix sort: LSD passes of 8 bits over (one key word, position) pairs; keys of
+// several words are packed into one when their significant bits fit 64, else
+// sorted word by word through the positions, and the keys and payloads are
+// gathered once at the end.
+//   * Up to kSmallSort keys: one block sorts them in shared memory, one launch
+//     for all passes (a pass is about 1 us there; through the grid its three
+//     launches alone take longer).
+//   * More: per pass k_radix_hist counts the digits of each tile of 4096 keys
+//     (warp-aggregated with __match_any_sync), k_radix_rows prefix-sums every
+//     digit's row of tile counts, and k_radix_scatter ranks every key inside
+//     its tile -- each warp walks its keys in rounds of 32 in input order, a
+//     key's rank is the count of its digit in earlier rounds plus its lanes
+//     before it in the round, and warps are offset per digit --, orders the
+//     tile in shared memory and writes every digit's run with neighbouring
+//     lanes (a pass moves 2 (key + 4) bytes per key; unordered stores cost it
+//     twice that in partial sectors).
+// Equal digits keep their input order, so the passes compose into a stable
+// sort.  Measured per pass, 4.35e6 (u64, u32) pairs: SORTTIMES.
 //
 // Scan: three phases over tiles of 2048 items (tile sums, one-block scan of
-// the tile sums, tile scans from their offsets).  Every phase reads its
-// items before it writes, so in == out is allowed.
+// the tile sums, tile scans from their offsets), or one block that carries its
+// sum from tile to tile when there are at most kScanTiles.  Every phase reads
+// its items before it writes, so in == out is allowed.
 #pragma once
 
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -133,6 +145,36 @@ __global__ void __launch_bounds__(kThreads) k_scan_tiles(const Tin* in, Tout* ou
 
 inline i64 tiles_of(i64 n) { return (n + kTile - 1) / kTile; }
 
+// A few tiles by one block: three launches take longer than its tile after
+// tile (about 1.2 us each) up to there.
+constexpr i64 kScanTiles = 4;
+template <class Tin, class Tout, bool Inclusive>
+__global__ void __launch_bounds__(kThreads) k_scan_few(const Tin* in, Tout* out, i64 n) {
+    __shared__ Tout tot;
+    Tout carry = 0;
+    for (i64 b = 0; b < n; b += kTile) {
+        const i64 base = b + (i64)threadIdx.x * kItems;
+        Tout v[kItems];
+        Tout sum = 0;
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) {
+            const i64 p = base + i;
+            v[i] = p < n ? (Tout)in[p] : Tout(0);
+            sum += v[i];
+        }
+        Tout run = carry + block_exclusive<Tout>(sum, &tot);
+        carry += tot;
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) {
+            const i64 p = base + i;
+            if (Inclusive) run += v[i];
+            if (p < n) out[p] = run;
+            if (!Inclusive) run += v[i];
+        }
+        __syncthreads();   // tot is read before the next tile writes it
+    }
+}
+
 // Temporary bytes of a scan of n items with Tout sums.
 template <class Tout>
 inline size_t scan_tmp_bytes(i64 n) {
@@ -145,6 +187,11 @@ template <class Tin, class Tout, bool Inclusive = false>
 void scan(const Tin* in, Tout* out, i64 n, cudaStream_t s, void* tmp = nullptr) {
     if (n <= 0) return;
     const i64 nt = tiles_of(n);
+    if (nt <= kScanTiles) {
+        k_scan_few<Tin, Tout, Inclusive><<<1, kThreads, 0, s>>>(in, out, n);
+        DNQ_CHECK_LAUNCH();
+        return;
+    }
     DBuf<Tout> own;
     Tout* sums = static_cast<Tout*>(tmp);
     if (!sums) {
@@ -191,23 +238,133 @@ struct RadixKey<ulonglong2> {
     }
 };
 
+// The digits of a sort: (word, shift) of every pass, least significant first.
+constexpr int kMaxPasses = 40;
+struct RadixPasses {
+    int n = 0;
+    unsigned char word[kMaxPasses], shift[kMaxPasses];
+    // 8-bit windows over the set bits of `mask` in word w
+    void add(int w, u64 mask) {
+        while (mask) {
+            const int sh = __builtin_ctzll(mask);
+            require(n < kMaxPasses, DNQ_ERR_INVALID, "too many radix passes");
+            word[n] = (unsigned char)w;
+            shift[n] = (unsigned char)sh;
+            ++n;
+            mask &= sh + 8 >= 64 ? 0ull : ~0ull << (sh + 8);
+        }
+    }
+};
+
+// Word i of key p, narrowed to the word type of its passes.
 template <class K>
-__device__ __forceinline__ u32 digit_of(const K& k, int word, int shift) {
-    return (u32)(RadixKey<K>::word(k, word) >> shift) & 0xffu;
+__device__ __forceinline__ u64 key_word(const K* k, i64 p, int w) {
+    return RadixKey<K>::word(k[p], w);
 }
 
-template <class K>
-__global__ void __launch_bounds__(kThreads) k_radix_hist(const K* keys, i64 n, int word,
-                                                         int shift, u32* hist, i64 ntiles) {
+constexpr int kSmallThreads = 512;
+constexpr int kSmallItems = 7;
+constexpr int kSmallSort = kSmallThreads * kSmallItems;   // 3584 keys: 45 KB shared
+constexpr int kSmallWarps = kSmallThreads / 32;
+
+// All passes of up to kSmallSort keys.  The current word of every key stays
+// at its input place in shared memory; the passes permute the places.
+template <class K, class P>
+__global__ void __launch_bounds__(kSmallThreads)
+k_radix_small(const K* kin, const P* pin, K* kout, P* pout, int n, RadixPasses R) {
+    __shared__ u64 sk[kSmallSort];
+    __shared__ u16 si[kSmallSort];
+    __shared__ u16 wh[kSmallWarps][256];
+    __shared__ u32 dsum[8];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int base = w * (kSmallItems * 32) + lane;
+    u16 at[kSmallItems];   // input place of this thread's items
+#pragma unroll
+    for (int i = 0; i < kSmallItems; ++i) at[i] = (u16)(base + 32 * i);
+    int cur = -1;
+    for (int q = 0; q < R.n; ++q) {
+        const int word = R.word[q], shift = R.shift[q];
+        if (word != cur) {
+            cur = word;
+            for (int p = tid; p < n; p += kSmallThreads) sk[p] = key_word(kin, p, word);
+        }
+        for (int t = tid; t < kSmallWarps * 128; t += kSmallThreads)
+            reinterpret_cast<u32*>(&wh[0][0])[t] = 0u;
+        __syncthreads();
+        u32 dg[kSmallItems], rk[kSmallItems];
+#pragma unroll
+        for (int i = 0; i < kSmallItems; ++i) {
+            const bool ok = base + 32 * i < n;
+            dg[i] = ok ? (u32)(sk[at[i]] >> shift) & 0xffu : 256u;
+            const unsigned m = __match_any_sync(0xffffffffu, dg[i]);
+            const u32 before = ok ? wh[w][dg[i]] : 0u;
+            rk[i] = before + __popc(m & lt_mask());
+            __syncwarp();
+            if (ok && (m & lt_mask()) == 0) wh[w][dg[i]] = (u16)(before + __popc(m));
+            __syncwarp();
+        }
+        __syncthreads();
+        u32 tot = 0, incl = 0;
+        if (tid < 256) {   // per digit: warps' counts -> offsets in the digit
+#pragma unroll
+            for (int k = 0; k < kSmallWarps; ++k) {
+                const u32 t = wh[k][tid];
+                wh[k][tid] = (u16)tot;
+                tot += t;
+            }
+            incl = tot;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const u32 y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            if (lane == 31) dsum[w] = incl;
+        }
+        __syncthreads();
+        if (tid < 256) {   // start of the digit
+            u32 st = incl - tot;
+            for (int k = 0; k < w; ++k) st += dsum[k];
+#pragma unroll
+            for (int k = 0; k < kSmallWarps; ++k) wh[k][tid] = (u16)(wh[k][tid] + st);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kSmallItems; ++i)
+            if (dg[i] < 256u) si[wh[w][dg[i]] + rk[i]] = at[i];
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kSmallItems; ++i)
+            if (base + 32 * i < n) at[i] = si[base + 32 * i];
+    }
+#pragma unroll
+    for (int i = 0; i < kSmallItems; ++i) {
+        const int p = base + 32 * i;
+        if (p >= n) continue;
+        if (kout) kout[p] = kin[at[i]];
+        if (pout) pout[p] = pin ? pin[at[i]] : (P)at[i];
+    }
+}
+
+constexpr int kRadixItems = 16;
+constexpr int kRadixTile = kThreads * kRadixItems;   // 4096
+
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_radix_hist(const T* keys, i64 n, int shift,
+                                                         u32* hist, i64 ntiles) {
     __shared__ u32 h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
-    const i64 base = (i64)blockIdx.x * kTile;
+    const i64 base = (i64)blockIdx.x * kRadixTile;
+    T k[kRadixItems];
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
+    for (int i = 0; i < kRadixItems; ++i) {
         const i64 p = base + (i64)i * kThreads + threadIdx.x;
-        const bool ok = p < n;
-        const u32 d = ok ? digit_of(keys[p], word, shift) : 256u;
+        k[i] = p < n ? keys[p] : T(0);
+    }
+#pragma unroll
+    for (int i = 0; i < kRadixItems; ++i) {
+        const bool ok = base + (i64)i * kThreads + threadIdx.x < n;
+        const u32 d = ok ? (u32)(k[i] >> shift) & 0xffu : 256u;
         const unsigned m = __match_any_sync(0xffffffffu, d);
         if (ok && (m & lt_mask()) == 0) atomicAdd(&h[d], (u32)__popc(m));
     }
@@ -215,56 +372,115 @@ __global__ void __launch_bounds__(kThreads) k_radix_hist(const K* keys, i64 n, i
     hist[(i64)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
-// Payload pass-through: P* may be null on output (keys only); a null input
-// with an output gives the input positions (P = u32).
-template <class K, class P>
-__global__ void __launch_bounds__(kThreads)
-k_radix_scatter(const K* kin, const P* pin, K* kout, P* pout, i64 n, int word, int shift,
-                const u32* offs, i64 ntiles) {
-    __shared__ u32 wh[kWarps][256];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int t = threadIdx.x; t < kWarps * 256; t += kThreads) (&wh[0][0])[t] = 0;
-    __syncthreads();
-    const i64 base = (i64)blockIdx.x * kTile + (i64)w * (kItems * 32);
-    K k[kItems];
-    P pl[kItems];
-    u32 dg[kItems], rk[kItems];
+// Block d: exclusive prefix sums of digit d's tile counts, in place, and
+// their total.
+__global__ void __launch_bounds__(kThreads) k_radix_rows(u32* hist, i64 ntiles, u32* total) {
+    __shared__ u32 tot;
+    u32* row = hist + (i64)blockIdx.x * ntiles;
+    u32 carry = 0;
+    for (i64 c0 = 0; c0 < ntiles; c0 += kThreads * 4) {
+        u32 v[4], sum = 0;
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        const i64 p = base + (i64)i * 32 + lane;
-        const bool ok = p < n;
-        dg[i] = 256u;
-        if (ok) {
-            k[i] = kin[p];
-            if (pout) pl[i] = pin ? pin[p] : (P)p;
-            dg[i] = digit_of(k[i], word, shift);
+        for (int i = 0; i < 4; ++i) {
+            const i64 p = c0 + (i64)threadIdx.x * 4 + i;
+            v[i] = p < ntiles ? row[p] : 0u;
+            sum += v[i];
         }
-        const unsigned m = __match_any_sync(0xffffffffu, dg[i]);
-        const u32 before = ok ? wh[w][dg[i]] : 0u;
-        rk[i] = before + __popc(m & lt_mask());
+        u32 run = carry + block_exclusive<u32>(sum, &tot);
+        carry += tot;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const i64 p = c0 + (i64)threadIdx.x * 4 + i;
+            if (p < ntiles) row[p] = run;
+            run += v[i];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) total[blockIdx.x] = carry;
+}
+
+// One pass.  pin == null gives each key's place; pout == null moves keys only.
+template <class T>
+__global__ void __launch_bounds__(kThreads)
+k_radix_scatter(const T* kin, const u32* pin, T* kout, u32* pout, i64 n, int shift,
+                const u32* offs, const u32* total, i64 ntiles) {
+    __shared__ T stage[kRadixTile];
+    __shared__ u16 wh[kWarps][256];
+    __shared__ u32 dst[256];   // global place of the digit's first key, less its place in the tile
+    __shared__ u32 tot;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int t = threadIdx.x; t < kWarps * 128; t += kThreads)
+        reinterpret_cast<u32*>(&wh[0][0])[t] = 0u;
+    const i64 tile0 = (i64)blockIdx.x * kRadixTile;
+    const int m_tile = (int)min((i64)kRadixTile, n - tile0);
+    const int base = w * (kRadixItems * 32) + lane;
+    T k[kRadixItems];
+#pragma unroll
+    for (int i = 0; i < kRadixItems; ++i)
+        k[i] = base + 32 * i < m_tile ? kin[tile0 + base + 32 * i] : T(0);
+    __syncthreads();
+    u16 rk[kRadixItems];
+#pragma unroll
+    for (int i = 0; i < kRadixItems; ++i) {
+        const bool ok = base + 32 * i < m_tile;
+        const u32 d = ok ? (u32)(k[i] >> shift) & 0xffu : 256u;
+        const unsigned m = __match_any_sync(0xffffffffu, d);
+        const u32 before = ok ? wh[w][d] : 0u;
+        rk[i] = (u16)(before + __popc(m & lt_mask()));
         __syncwarp();
-        if (ok && (m & lt_mask()) == 0) wh[w][dg[i]] = before + __popc(m);
+        if (ok && (m & lt_mask()) == 0) wh[w][d] = (u16)(before + __popc(m));
         __syncwarp();
     }
     __syncthreads();
-    {   // per digit: warps' counts -> exclusive offsets
+    {   // per digit: warps' counts -> places in the tile, and where it goes
         const int d = threadIdx.x;
         u32 acc = 0;
 #pragma unroll
         for (int q = 0; q < kWarps; ++q) {
             const u32 t = wh[q][d];
-            wh[q][d] = acc;
+            wh[q][d] = (u16)acc;
             acc += t;
         }
+        const u32 start = block_exclusive<u32>(acc, &tot);       // in the tile
+        const u32 below = block_exclusive<u32>(total[d], &tot);  // keys of lower digits
+#pragma unroll
+        for (int q = 0; q < kWarps; ++q) wh[q][d] = (u16)(wh[q][d] + start);
+        dst[d] = below + offs[(i64)d * ntiles + blockIdx.x] - start;
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        if (dg[i] < 256u) {
-            const u32 pos = offs[(i64)dg[i] * ntiles + blockIdx.x] + wh[w][dg[i]] + rk[i];
-            kout[pos] = k[i];
-            if (pout) pout[pos] = pl[i];
-        }
+    for (int i = 0; i < kRadixItems; ++i) {
+        if (base + 32 * i >= m_tile) continue;
+        rk[i] = (u16)(rk[i] + wh[w][(u32)(k[i] >> shift) & 0xffu]);   // place in the tile
+        stage[rk[i]] = k[i];
+    }
+    __syncthreads();
+    u32 to[kRadixItems];
+#pragma unroll
+    for (int i = 0; i < kRadixItems; ++i) {
+        const int l = i * kThreads + threadIdx.x;
+        if (l >= m_tile) continue;
+        const T key = stage[l];
+        to[i] = dst[(u32)(key >> shift) & 0xffu] + (u32)l;
+        kout[to[i]] = key;
+    }
+    if (!pout) return;
+    u32 pl[kRadixItems];
+#pragma unroll
+    for (int i = 0; i < kRadixItems; ++i) {
+        const i64 p = tile0 + base + 32 * i;
+        if (base + 32 * i < m_tile) pl[i] = pin ? pin[p] : (u32)p;
+    }
+    __syncthreads();
+    u32* sp = reinterpret_cast<u32*>(stage);
+#pragma unroll
+    for (int i = 0; i < kRadixItems; ++i)
+        if (base + 32 * i < m_tile) sp[rk[i]] = pl[i];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kRadixItems; ++i) {
+        const int l = i * kThreads + threadIdx.x;
+        if (l < m_tile) pout[to[i]] = sp[l];
     }
 }
 
@@ -277,50 +493,125 @@ __global__ void k_copy_pairs(const K* kin, const P* pin, K* kout, P* pout, i64 n
     }
 }
 
-// Stable sort of n (key, payload) pairs by key, ascending; n < 2^32.
-// bits[i] = significant low bits of key word i (most significant word
-// first; the other bits of the word must be zero, or at least equal in all
-// keys).  pout == null sorts keys only; pin == null with a payload output
-// gives each key's input position.  kin != kout.
-template <class K, class P>
-void radix_sort(const K* kin, K* kout, const P* pin, P* pout, i64 n, const int* bits,
-                cudaStream_t s) {
-    if (n <= 0) return;
-    require(n < (i64)0xffffffffll, DNQ_ERR_OVERFLOW, "radix sort of 2^32 or more keys");
-    constexpr int W = RadixKey<K>::W;
-    int pw[16 * W], ps[16 * W], np = 0;
-    for (int i = W - 1; i >= 0; --i)      // least significant word first
-        for (int sh = 0; sh < bits[i]; sh += 8) {
-            pw[np] = i;
-            ps[np] = sh;
-            ++np;
-        }
-    const unsigned grid_copy = (unsigned)std::min<i64>((n + 255) / 256, 4096);
-    if (np == 0) {
-        k_copy_pairs<K, P><<<grid_copy, 256, 0, s>>>(kin, pin, kout, pout, n);
-        DNQ_CHECK_LAUNCH();
-        return;
+// out[t] = word w of key at[t] (at == null: key t); with w < 0 all words of a
+// two-word key packed as word 0 << lo_bits | word 1, both masked.
+template <class K>
+__global__ void k_radix_word(const K* k, const u32* at, i64 n, int w, int hi_bits, int lo_bits,
+                             u64* out) {
+    for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
+         t += (i64)gridDim.x * blockDim.x) {
+        const i64 p = at ? (i64)at[t] : t;
+        out[t] = w >= 0 ? key_word(k, p, w)
+                        : ((key_word(k, p, 0) & low_mask(hi_bits)) << lo_bits) |
+                              (key_word(k, p, 1) & low_mask(lo_bits));
     }
-    const i64 nt = tiles_of(n);
-    DBuf<K> kt(np > 1 ? n : 0, s);
-    DBuf<P> pt((np > 1 && pout) ? n : 0, s);
-    DBuf<u32> hist(256 * nt, s);
-    DBuf<u32> stmp(tiles_of(256 * nt), s);
-    const K* ksrc = kin;
-    const P* psrc = pin;
-    for (int q = 0; q < np; ++q) {
-        const bool to_out = ((np - 1 - q) & 1) == 0;
-        K* kdst = to_out ? kout : kt.p;
-        P* pdst = pout ? (to_out ? pout : pt.p) : nullptr;
-        k_radix_hist<K><<<(unsigned)nt, kThreads, 0, s>>>(ksrc, n, pw[q], ps[q], hist.p, nt);
+}
+
+template <class K, class P>
+__global__ void k_radix_gather(const K* kin, const P* pin, const u32* at, i64 n, K* kout,
+                               P* pout) {
+    for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
+         t += (i64)gridDim.x * blockDim.x) {
+        const u32 p = at[t];
+        kout[t] = kin[p];
+        if (pout) pout[t] = pin ? pin[p] : (P)p;
+    }
+}
+
+// The passes of R (one word) over n (key, u32) pairs; the result ends in
+// kout / pout (pout null: keys only).
+template <class T>
+void radix_passes(const T* kin, const u32* pin, T* kout, u32* pout, i64 n, const RadixPasses& R,
+                  cudaStream_t s) {
+    const i64 nt = (n + kRadixTile - 1) / kRadixTile;
+    DBuf<T> kt(R.n > 1 ? n : 0, s);
+    DBuf<u32> pt((R.n > 1 && pout) ? n : 0, s);
+    DBuf<u32> hist(256 * nt, s), total(256, s);
+    const T* ksrc = kin;
+    const u32* psrc = pin;
+    for (int q = 0; q < R.n; ++q) {
+        const bool to_out = ((R.n - 1 - q) & 1) == 0;
+        T* kdst = to_out ? kout : kt.p;
+        u32* pdst = pout ? (to_out ? pout : pt.p) : nullptr;
+        k_radix_hist<T><<<(unsigned)nt, kThreads, 0, s>>>(ksrc, n, R.shift[q], hist.p, nt);
         DNQ_CHECK_LAUNCH();
-        scan<u32, u32, false>(hist.p, hist.p, 256 * nt, s, stmp.p);
-        k_radix_scatter<K, P><<<(unsigned)nt, kThreads, 0, s>>>(ksrc, psrc, kdst, pdst, n,
-                                                                pw[q], ps[q], hist.p, nt);
+        k_radix_rows<<<256, kThreads, 0, s>>>(hist.p, nt, total.p);
+        DNQ_CHECK_LAUNCH();
+        k_radix_scatter<T><<<(unsigned)nt, kThreads, 0, s>>>(ksrc, psrc, kdst, pdst, n,
+                                                             R.shift[q], hist.p, total.p, nt);
         DNQ_CHECK_LAUNCH();
         ksrc = kdst;
         psrc = pdst;
     }
+}
+
+// Stable sort of n (key, payload) pairs by key, ascending; n < 2^32.
+// mask[i] = significant bits of key word i (most significant word first; the
+// other bits of the word must be equal in all keys).  pout == null sorts keys
+// only; pin == null with a payload output gives each key's input position.
+// kin != kout.
+template <class K, class P>
+void radix_sort_masked(const K* kin, K* kout, const P* pin, P* pout, i64 n, const u64* mask,
+                       cudaStream_t s) {
+    if (n <= 0) return;
+    require(n < (i64)0xffffffffll, DNQ_ERR_OVERFLOW, "radix sort of 2^32 or more keys");
+    constexpr int W = RadixKey<K>::W;
+    const unsigned grid = (unsigned)std::min<i64>((n + 255) / 256, 1 << 20);
+    RadixPasses all;
+    for (int i = W - 1; i >= 0; --i) all.add(i, mask[i]);   // least significant word first
+    if (all.n == 0) {
+        k_copy_pairs<K, P><<<grid, 256, 0, s>>>(kin, pin, kout, pout, n);
+        DNQ_CHECK_LAUNCH();
+        return;
+    }
+    if (n <= kSmallSort) {
+        k_radix_small<K, P><<<1, kSmallThreads, 0, s>>>(kin, pin, kout, pout, (int)n, all);
+        DNQ_CHECK_LAUNCH();
+        return;
+    }
+    if constexpr (W == 1) {
+        if constexpr (std::is_same<P, u32>::value) {
+            radix_passes<K>(kin, pin, kout, pout, n, all, s);
+            return;
+        }
+    }
+    // several words, or another payload: positions by one word after the other
+    DBuf<u32> at(n, s), at2(n, s);
+    DBuf<u64> kw(n, s), kw2(n, s);
+    u32 *cur = nullptr, *next = at.p;
+    auto by_word = [&](int w, int hi_bits, int lo_bits, u64 m) {
+        if (!m) return;
+        RadixPasses R;
+        R.add(0, m);
+        k_radix_word<K><<<grid, 256, 0, s>>>(kin, cur, n, w, hi_bits, lo_bits, kw.p);
+        DNQ_CHECK_LAUNCH();
+        radix_passes<u64>(kw.p, cur, kw2.p, next, n, R, s);
+        cur = next;
+        next = cur == at.p ? at2.p : at.p;
+    };
+    int hb = 0, lb = 0;
+    if constexpr (W == 2) {
+        hb = mask[0] ? 64 - __builtin_clzll(mask[0]) : 0;
+        lb = mask[1] ? 64 - __builtin_clzll(mask[1]) : 0;
+    }
+    if (W == 2 && hb && lb && hb + lb <= 64) {
+        by_word(-1, hb, lb, low_mask(hb + lb));
+    } else {
+        for (int i = W - 1; i >= 0; --i) by_word(i, 0, 0, mask[i]);
+    }
+    kw.release();
+    kw2.release();
+    k_radix_gather<K, P><<<grid, 256, 0, s>>>(kin, pin, cur, n, kout, pout);
+    DNQ_CHECK_LAUNCH();
+}
+
+// The same with bits[i] = significant low bits of key word i.
+template <class K, class P>
+void radix_sort(const K* kin, K* kout, const P* pin, P* pout, i64 n, const int* bits,
+                cudaStream_t s) {
+    u64 mask[RadixKey<K>::W];
+    for (int i = 0; i < RadixKey<K>::W; ++i) mask[i] = low_mask(bits[i]);
+    radix_sort_masked<K, P>(kin, kout, pin, pout, n, mask, s);
 }
 
 // ---------------------------------------------------------------------------

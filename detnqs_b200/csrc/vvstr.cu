@@ -97,12 +97,11 @@ struct StrIndex {
     StrMapView view() const { return StrMapView{slots.p, mask}; }
 };
 
-__global__ void k_keys_by(const u64* V, i64 n, int major, ulonglong2* k, u32* id) {
+__global__ void k_keys_by(const u64* V, i64 n, int major, ulonglong2* k) {
     for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
          t += (i64)gridDim.x * blockDim.x) {
         const u64 a = V[2 * t], b = V[2 * t + 1];
         k[t] = major == 0 ? make_ulonglong2(a, b) : make_ulonglong2(b, a);
-        id[t] = (u32)t;
     }
 }
 
@@ -150,12 +149,11 @@ __global__ void k_len_hist(const u32* gstart, const u32* ngroups, i64 nmax, u32*
 }
 
 // Strings of at most 32 orbitals: one 64-bit key (group string << 32 | companion).
-__global__ void k_keys_by64(const u64* V, i64 n, int major, u64* k, u32* id) {
+__global__ void k_keys_by64(const u64* V, i64 n, int major, u64* k) {
     for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
          t += (i64)gridDim.x * blockDim.x) {
         const u64 a = V[2 * t], b = V[2 * t + 1];
         k[t] = major == 0 ? (a << 32) | b : (b << 32) | a;
-        id[t] = (u32)t;
     }
 }
 
@@ -228,7 +226,6 @@ void str_index_begin(StrIndex& X, const u64* V, i64 n, int major, int n_orb, Ind
     const bool narrow = n_orb <= 32;
     DBuf<ulonglong2> k;
     DBuf<u64> k64;
-    DBuf<u32> id(n, s);
     X.idx.alloc(n, s);
     X.other.alloc(n, s);
     DBuf<unsigned> head(n, s);
@@ -237,19 +234,19 @@ void str_index_begin(StrIndex& X, const u64* V, i64 n, int major, int n_orb, Ind
         k64.alloc(n, s);
         X.ks64.alloc(n, s);
         X.other32.alloc(n, s);
-        k_keys_by64<<<gsz(n), 256, 0, s>>>(V, n, major, k64.p, id.p);
+        k_keys_by64<<<gsz(n), 256, 0, s>>>(V, n, major, k64.p);
         DNQ_CHECK_LAUNCH();
-        const int bits[1] = {32 + n_orb};
-        prim::radix_sort<u64, u32>(k64.p, X.ks64.p, id.p, X.idx.p, n, bits, s);
+        const u64 mask[1] = {low_mask(n_orb) << 32 | low_mask(n_orb)};
+        prim::radix_sort_masked<u64, u32>(k64.p, X.ks64.p, nullptr, X.idx.p, n, mask, s);
         k_split_sorted64<<<gsz(n), 256, 0, s>>>(X.ks64.p, n, X.other.p, X.other32.p, head.p, dup);
         DNQ_CHECK_LAUNCH();
     } else {
         k.alloc(n, s);
         X.ks.alloc(n, s);
-        k_keys_by<<<gsz(n), 256, 0, s>>>(V, n, major, k.p, id.p);
+        k_keys_by<<<gsz(n), 256, 0, s>>>(V, n, major, k.p);
         DNQ_CHECK_LAUNCH();
         const int bits[2] = {n_orb, n_orb};
-        prim::radix_sort<ulonglong2, u32>(k.p, X.ks.p, id.p, X.idx.p, n, bits, s);
+        prim::radix_sort<ulonglong2, u32>(k.p, X.ks.p, nullptr, X.idx.p, n, bits, s);
         k_split_sorted<<<gsz(n), 256, 0, s>>>(X.ks.p, n, X.other.p, head.p, dup);
         DNQ_CHECK_LAUNCH();
     }
