@@ -329,7 +329,9 @@ void to_f32(const double* x, i64 n, float* o, cudaStream_t s) {
 
 void energy_reduce(const double* x, const double* y, i64 n, double* eloc, double* out2_dev,
                    cudaStream_t s) {
-    const int nb = 592;
+    // blocks past n / 256 would hold nothing: their zero partials do not change
+    // the sums, but merging 592 takes one thread 23 us
+    const int nb = (int)std::min<i64>(592, (n + 255) / 256);
     DBuf<double> part(4 * nb, s);
     k_energy_partials<<<nb, 256, 0, s>>>(x, y, n, eloc, part.p);
     DNQ_CHECK_LAUNCH();

@@ -582,10 +582,12 @@ struct Arena {
     u32* big;                         // rows longer than one chunk
     u32* big_len;                     // their member counts
     int* n_big;
+    uint2* unit;                      // 64-member units of the long rows: (place in big, unit)
+    unsigned long long* n_unit;
     int* next_row;
     const u32* order;                 // walk order of the rows (null: 0, 1, ...)
     unsigned long long* n_test;
-    unsigned long long* n_hit;        // members recorded by k_vv_arena (optional)
+    unsigned long long* n_hit;        // members recorded by k_vv_arena
     // single excitations recorded by k_vv_arena in warp-private slices of
     // sgl_slice entries, evaluated by k_vv_singles one per thread; past its
     // slice a warp leaves them ordinary members
@@ -1487,7 +1489,7 @@ __global__ void __launch_bounds__(kWS * 32, 3) k_vv_arena(Loc L, Arena A) {
     }
     if (lane == 0) {
         atomicAdd(A.n_test, tests);
-        if (A.n_hit) atomicAdd(A.n_hit, hits);
+        atomicAdd(A.n_hit, hits);
         if (A.sgl) A.sgl_n[wid] = sgn < A.sgl_slice ? sgn : A.sgl_slice;
     }
 }
@@ -1521,7 +1523,11 @@ __global__ void __launch_bounds__(256) k_vv_singles(Loc L, Arena A) {
 // Single pass, second half: the members of every arena row become its
 // entries, in place and in order (a step reads its 64 members before it
 // writes, and writes only at positions below the next step's).  One warp
-// per row, all lanes evaluating.
+// per row, all lanes evaluating.  A row of more than kLongEval members and
+// twice a warp's share of all members would be the kernel's tail (a row
+// connected to most of a small space took 60 of 67 us at 2,241 rows): it
+// joins the rows that k_vv_eval_long spreads over the grid.
+constexpr unsigned long long kLongEval = 512;
 template <class Loc>
 __global__ void __launch_bounds__(kWS * 32) k_vv_eval(Loc L, Arena A) {
     const int lane = threadIdx.x & 31;
@@ -1530,10 +1536,16 @@ __global__ void __launch_bounds__(kWS * 32) k_vv_eval(Loc L, Arena A) {
     const i64 nrows = L.rows();
     if (*(volatile int*)A.overflow) return;
     const u64* mem = reinterpret_cast<const u64*>(A.aval);
+    const unsigned long long share = 2 * *A.n_hit / (unsigned long long)nw;
+    const unsigned long long most = share > kLongEval ? share : kLongEval;
     for (i64 g = gw; g < nrows; g += nw) {
         const i64 pos = A.row_pos[g];
-        if (pos < 0) continue;   // a long row
+        if (pos < 0) continue;   // a row longer than a chunk
         const u32 len = A.row_len[g];
+        if (len > most) {
+            if (lane == 0) A.big[atomicAdd(A.n_big, 1)] = (u32)g;
+            continue;
+        }
         int r;
         u32 cb;
         const VVParams& P = L.at(g, r, cb);
@@ -1573,10 +1585,11 @@ __global__ void __launch_bounds__(kWS * 32) k_vv_eval(Loc L, Arena A) {
     }
 }
 
-// Rows longer than a chunk: exact contiguous space and a second walk that
-// records their members there (one warp per row; the walk is cheap next to
-// the evaluation, which k_vv_eval_long spreads over the whole grid).  The
-// count of such rows is read on the device so the launch can sit in a graph.
+// The long rows.  One longer than a chunk gets exact contiguous space and a
+// second walk that records its members there (one warp per row; the walk is
+// cheap next to the evaluation); one left by k_vv_eval has its members in
+// place.  Their 64-member units are listed for k_vv_eval_long.  The count of
+// such rows is read on the device so the launch can sit in a graph.
 template <class Loc, class W>
 __global__ void __launch_bounds__(kWS * 32) k_vv_big(Loc L, Arena A) {
     __shared__ WarpShared sh[kWS];
@@ -1589,53 +1602,60 @@ __global__ void __launch_bounds__(kWS * 32) k_vv_big(Loc L, Arena A) {
     for (int i = gw; i < nbig; i += nw) {
         const int g = (int)A.big[i];
         const u32 len = A.row_len[g];
-        unsigned long long base = 0;   // 4-slot multiples keep every start aligned
-        if (lane == 0) base = atomicAdd(A.cursor, (unsigned long long)((len + 3u) & ~3u));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if ((i64)base + len > A.cap) {
-            if (lane == 0) atomicExch(A.overflow, 1);
-            continue;
+        i64 pos = A.row_pos[g];
+        if (pos < 0) {
+            unsigned long long base = 0;   // 4-slot multiples keep every start aligned
+            if (lane == 0)
+                base = atomicAdd(A.cursor, (unsigned long long)((len + 3u) & ~3u));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if ((i64)base + len > A.cap) {
+                if (lane == 0) atomicExch(A.overflow, 1);
+                continue;
+            }
+            pos = (i64)base;
+            int r;
+            u32 cb;
+            const VVParams& P = L.at(g, r, cb);
+            u64 a, b;
+            double psr, cut;
+            row_setup(P, r, a, b, psr, cut);
+            load_lists(S, a, b, P.n_orb);
+            HitOut out{reinterpret_cast<u64*>(A.aval) + pos, (u32)len};
+            unsigned long long tt = 0;
+            walk_any<W>(P, r, a, b, S, out, tt);
         }
-        int r;
-        u32 cb;
-        const VVParams& P = L.at(g, r, cb);
-        u64 a, b;
-        double psr, cut;
-        row_setup(P, r, a, b, psr, cut);
-        load_lists(S, a, b, P.n_orb);
-        HitOut out{reinterpret_cast<u64*>(A.aval) + base, (u32)len};
-        unsigned long long tt = 0;
-        walk_any<W>(P, r, a, b, S, out, tt);
+        const u32 units = (len + 63) / 64;
+        unsigned long long u0 = 0;
         if (lane == 0) {
-            A.row_pos[g] = (i64)base | kLongRow;
+            A.row_pos[g] = pos | kLongRow;
             A.big_len[i] = len;
             A.row_len[g] = 0;   // entries kept, summed by k_vv_eval_long
+            u0 = atomicAdd(A.n_unit, (unsigned long long)units);
         }
+        u0 = __shfl_sync(0xffffffffu, u0, 0);
+        for (u32 u = lane; u < units; u += 32) A.unit[u0 + u] = make_uint2((u32)i, u);
         __syncwarp();
     }
 }
 
-// The members of the long rows become entries in place, 64 per warp step
-// over the whole grid; a dropped member leaves a hole.  The 64-member units
-// of all long rows are dealt round-robin to the warps as one sequence (unit
-// u of row i goes to warp (units before row i + u) mod warps).  Kept counts
+// Units listed for rows in `slots` arena slots: whole ones and a last one each.
+inline i64 unit_bound(i64 slots, i64 nrows) { return slots / 64 + nrows + 1; }
+
+// The members of the long rows become entries in place, a 64-member unit per
+// warp step over the whole grid; a dropped member leaves a hole.  Kept counts
 // are summed into row_len.
 template <class Loc>
 __global__ void __launch_bounds__(kWS * 32) k_vv_eval_long(Loc L, Arena A) {
     const int lane = threadIdx.x & 31;
     const i64 gw = (blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5;
     const i64 nw = (gridDim.x * (i64)blockDim.x) >> 5;
-    const int nbig = *A.n_big;
     if (*(volatile int*)A.overflow) return;
+    const i64 nu = (i64)*A.n_unit;
     const u64* mem = reinterpret_cast<const u64*>(A.aval);
-    i64 off = 0;   // units of the rows before row i, mod nw
-    for (int i = 0; i < nbig; ++i) {
-        const int g = (int)A.big[i];
-        const i64 len = A.big_len[i];
-        const i64 units = (len + 63) / 64;
-        const i64 u0 = (gw - off + nw) % nw;   // this warp's first unit of row i
-        off = (off + units) % nw;
-        if (u0 >= units) continue;
+    for (i64 q = gw; q < nu; q += nw) {
+        const uint2 un = A.unit[q];
+        const int g = (int)A.big[un.x];
+        const i64 len = A.big_len[un.x];
         const i64 pos = A.row_pos[g] & ~kLongRow;
         int r;
         u32 cb;
@@ -1644,20 +1664,18 @@ __global__ void __launch_bounds__(kWS * 32) k_vv_eval_long(Loc L, Arena A) {
         double psr, cut;
         row_setup(P, r, a, b, psr, cut);
         u32 kept = 0;
-        for (i64 k0 = u0 * 64; k0 < len; k0 += nw * 64) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const i64 k = k0 + 32 * h + lane;
-                bool keep = false;
-                if (k < len) {
-                    const u64 m = mem[pos + k];
-                    const Hit e = eval_hit(P, r, a, b, psr, cut, (u32)m, (u32)(m >> 32));
-                    keep = e.keep;
-                    A.acol[pos + k] = e.keep ? e.j + cb : kHole;
-                    A.aval[pos + k] = e.h;
-                }
-                kept += __popc(__ballot_sync(0xffffffffu, keep));
+        for (int h = 0; h < 2; ++h) {
+            const i64 k = (i64)un.y * 64 + 32 * h + lane;
+            bool keep = false;
+            if (k < len) {
+                const u64 m = mem[pos + k];
+                const Hit e = eval_hit(P, r, a, b, psr, cut, (u32)m, (u32)(m >> 32), A.sres);
+                keep = e.keep;
+                A.acol[pos + k] = e.keep ? e.j + cb : kHole;
+                A.aval[pos + k] = e.h;
             }
+            kept += __popc(__ballot_sync(0xffffffffu, keep));
         }
         if (lane == 0 && kept) atomicAdd(&A.row_len[g], kept);
     }
@@ -1678,7 +1696,8 @@ __global__ void __launch_bounds__(256) k_vv_compact_long(const u32* big, const u
     for (int i = blockIdx.x; i < nbig; i += gridDim.x) {
         const u32 g = big[i];
         const i64 src = row_pos[g] & ~kLongRow, dst = rowptr[g];
-        const i64 len = big_len[i];
+        // a row without entries, or of a step whose row pointers were cleared
+        const i64 len = rowptr[g + 1] > dst ? (i64)big_len[i] : 0;
         if (val32 && threadIdx.x == 0) dg[g] = 0.0;   // set below when the row keeps it
         __syncthreads();
         i64 carry = 0;
@@ -1897,6 +1916,16 @@ i64 arena_bound(i64 nnz, i64 nrows, int grid, i64 chunk) {
     return nnz + nnz / 3 + 1 + 4 * nrows + ((i64)grid * kWS + 1) * chunk;
 }
 
+// Bytes the device's stream-ordered pool has mapped and not handed out.
+i64 pool_unused(int device) {
+    cudaMemPool_t pool;
+    DNQ_CUDA(cudaDeviceGetMemPool(&pool, device));
+    u64 reserved = 0, used = 0;
+    DNQ_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+    DNQ_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+    return reserved > used ? (i64)(reserved - used) : 0;
+}
+
 template <class Loc>
 int vv_grid(int device) {
     int per_sm = 0;
@@ -2006,8 +2035,6 @@ i64 run_vv(const Loc& L, i64 nrows, i64 cap_hint, int device, cudaStream_t s, Cs
     Events<4> ev;
     const int grid = vv_grid<Loc>(device);
     const i64 warps = (i64)grid * kWS;
-    size_t freeb = 0, totb = 0;
-    DNQ_CUDA(cudaMemGetInfo(&freeb, &totb));
     // chunks of whole 4-slot groups (row starts stay aligned)
     const i64 chunk = opt.arena_chunk > 0 ? ((i64)opt.arena_chunk + 3) & ~3ll
                       : nrows >= 64 * warps             ? kChunkLarge
@@ -2015,8 +2042,16 @@ i64 run_vv(const Loc& L, i64 nrows, i64 cap_hint, int device, cudaStream_t s, Cs
     i64 want = cap_hint > 0 ? cap_hint + cap_hint / 8 : 512 * nrows;
     want += warps * chunk;
     const bool f32_in_build = arena_out && dg;   // k_vv_eval writes the FP32 copy
-    const i64 maxfit = (i64)(freeb / 2 / (f32_in_build ? 16 : 12));
-    i64 cap = std::max<i64>(std::min(want, maxfit), chunk);
+    // at most half of the free memory; what the device's pool holds unused (as
+    // after an earlier build of this size) needs no look at that, which
+    // takes the driver 70 us, and 0.2-0.8 ms one time in ten
+    const i64 slot_bytes = f32_in_build ? 16 : 12;
+    i64 cap = std::max<i64>(want, chunk);
+    if (pool_unused(device) < cap * slot_bytes) {
+        size_t freeb = 0, totb = 0;
+        DNQ_CUDA(cudaMemGetInfo(&freeb, &totb));
+        cap = std::max<i64>(std::min(want, (i64)freeb / 2 / slot_bytes), chunk);
+    }
     if (opt.arena_cap > 0) cap = (i64)opt.arena_cap;
     DBuf<int> next(1, s), ovf(1, s), nbig(1, s), bad(1, s);
     DBuf<unsigned long long> nt(1, s), cursor(1, s), nh(1, s);
@@ -2036,7 +2071,11 @@ i64 run_vv(const Loc& L, i64 nrows, i64 cap_hint, int device, cudaStream_t s, Cs
         dg->alloc(nrows, s);
     }
     DBuf<i64> rpos(nrows, s);
+    DBuf<uint2> unit(unit_bound(cap, nrows), s);
+    DBuf<unsigned long long> nunit(1, s);
     Arena A{};
+    A.unit = unit.p;
+    A.n_unit = nunit.p;
     A.acol = acol.p;
     A.aval = aval.p;
     A.cap = cap;
@@ -2062,6 +2101,7 @@ i64 run_vv(const Loc& L, i64 nrows, i64 cap_hint, int device, cudaStream_t s, Cs
     A.dg = f32_in_build ? dg->p : nullptr;
     DNQ_CUDA(cudaMemsetAsync(nt.p, 0, 8, s));
     DNQ_CUDA(cudaMemsetAsync(nh.p, 0, 8, s));
+    DNQ_CUDA(cudaMemsetAsync(nunit.p, 0, 8, s));
     DNQ_CUDA(cudaMemsetAsync(next.p, 0, 4, s));
     DNQ_CUDA(cudaMemsetAsync(ovf.p, 0, 4, s));
     DNQ_CUDA(cudaMemsetAsync(nbig.p, 0, 4, s));
@@ -2105,7 +2145,6 @@ i64 run_vv(const Loc& L, i64 nrows, i64 cap_hint, int device, cudaStream_t s, Cs
         // the open-chunk reserve dominates) keeps only the handed-out prefix,
         // at the same offsets, so its H.psi reads the same slots.
         const i64 used = std::min<i64>((i64)hcur, cap);
-        const i64 slot_bytes = f32_in_build ? 16 : 12;
         if (used <= cap / 4 && (cap - used) * slot_bytes >= (64ll << 20)) {
             DBuf<u32> c2(used, s);
             DBuf<double> v2(used, s);
@@ -2778,7 +2817,8 @@ struct dnq_batch_s {
     dnq::DBuf<double> aval;
     dnq::DBuf<dnq::i64> rpos;
     dnq::DBuf<int> next, ovf, nbig, bad;
-    dnq::DBuf<unsigned long long> nt, cursor;
+    dnq::DBuf<unsigned long long> nt, nh, nunit, cursor;
+    dnq::DBuf<uint2> unit;
     dnq::DBuf<dnq::u8> scan_tmp;
     dnq::i64 cap = 0;
     dnq::i64 hits = 0;   // members of the sizing build (the arena holds members)
@@ -2862,6 +2902,9 @@ void plan(dnq_batch_s* b, cudaStream_t s) {
     b->nbig.alloc(1, s);
     b->bad.alloc(1, s);
     b->nt.alloc(1, s);
+    b->nh.alloc(1, s);
+    b->nunit.alloc(1, s);
+    b->unit.alloc(unit_bound(b->cap, n), s);
     b->cursor.alloc(1, s);
     b->val32.alloc(nnz, s);
     b->diag_op.alloc(n, s);
@@ -2923,6 +2966,9 @@ void enqueue_step(dnq_batch_s* b, int precision, cudaStream_t s, cudaEvent_t* ev
     A.n_big = b->nbig.p;
     A.next_row = b->next.p;
     A.n_test = b->nt.p;
+    A.n_hit = b->nh.p;
+    A.unit = b->unit.p;
+    A.n_unit = b->nunit.p;
     k_diag_batch<<<sm_count(b->device) * 4, 256, 0, s>>>(L, b->diag.p);
     DNQ_CHECK_LAUNCH();
     mark(1);
@@ -2930,6 +2976,8 @@ void enqueue_step(dnq_batch_s* b, int precision, cudaStream_t s, cudaEvent_t* ev
     DNQ_CUDA(cudaMemsetAsync(b->ovf.p, 0, 4, s));
     DNQ_CUDA(cudaMemsetAsync(b->nbig.p, 0, 4, s));
     DNQ_CUDA(cudaMemsetAsync(b->nt.p, 0, 8, s));
+    DNQ_CUDA(cudaMemsetAsync(b->nh.p, 0, 8, s));
+    DNQ_CUDA(cudaMemsetAsync(b->nunit.p, 0, 8, s));
     DNQ_CUDA(cudaMemsetAsync(b->cursor.p, 0, 8, s));
     DNQ_CUDA(cudaMemsetAsync(b->bad.p, 0, 4, s));
     DNQ_CUDA(cudaMemsetAsync(b->rlen.p + n, 0, 4, s));
@@ -3141,6 +3189,7 @@ int dnq_batch_set_config(dnq_batch_t b, const int64_t* cfg4) {
         b->cap = arena_bound(std::max(b->M.nnz, b->hits), b->total, grid, b->chunk);
         b->acol.alloc(b->cap, nullptr);
         b->aval.alloc(b->cap, nullptr);
+        b->unit.alloc(unit_bound(b->cap, b->total), nullptr);
         DNQ_CUDA(cudaStreamSynchronize(nullptr));
     }
     b->drop_graphs();
