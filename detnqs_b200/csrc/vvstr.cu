@@ -444,11 +444,15 @@ void presence_rows(StrIndex& A, const StrIndex& B, i64 n, u32 thr, unsigned long
     A.pres_min = thr;
 }
 
-__device__ __forceinline__ i64 tri2(i64 p, i64 q) {
-    return p >= q ? p * (p + 1) / 2 + q : q * (q + 1) / 2 + p;
+// Packed triangular index of a pair; with at most 64 orbitals the ERI index
+// stays below 2,163,241, so 32 bits do.
+__device__ __forceinline__ u32 tri2(u32 p, u32 q) {
+    const u32 hi = max(p, q), lo = min(p, q);
+    return (hi * (hi + 1u) >> 1) + lo;
 }
-__device__ __forceinline__ double eri(const double* E, int p, int q, int r, int s) {
-    return __ldg(&E[tri2(tri2(p, q), tri2(r, s))]);
+// (pq|rs) from the keys of its pairs.
+__device__ __forceinline__ double eri(const double* E, u32 pq, u32 rs) {
+    return __ldg(&E[tri2(pq, rs)]);
 }
 
 // Part C costs of every group of index X (one warp per group): the walk of
@@ -675,28 +679,37 @@ struct ExactOut {
     }
 };
 
+// Strings are handled as W: u32 when every string of the system fits in 32
+// orbitals (half the bytes and instructions), else u64.
+__device__ __forceinline__ int popc_w(u32 x) { return __popc(x); }
+__device__ __forceinline__ int popc_w(u64 x) { return __popcll(x); }
+__device__ __forceinline__ int low_w(u32 x) { return __ffs(x) - 1; }
+__device__ __forceinline__ int low_w(u64 x) { return __ffsll(x) - 1; }
+__device__ __forceinline__ int high_w(u32 x) { return 31 - __clz(x); }
+__device__ __forceinline__ int high_w(u64 x) { return 63 - __clzll((long long)x); }
+
+// Occupied orbitals of occ strictly between two different orbitals.
+template <class W>
+__device__ __forceinline__ int between_w(W occ, int p, int q) {
+    const int lo = min(p, q), hi = max(p, q);
+    return popc_w((W)(occ & (((W)1 << hi) - ((W)2 << lo))));
+}
+
 // Single within one spin: bra string x -> ket string y (differ in 2 bits).
-__device__ __forceinline__ double str_single(const VVParams& P, u64 a, u64 b, int spin, u64 x,
-                                             u64 y) {
-    const u64 d = x ^ y;
-    const int h = __ffsll(x & d) - 1;   // bra orbital
-    const int p = __ffsll(y & d) - 1;   // ket orbital
-    return single_elem(P.C, a, b, spin, h, p);
+template <class W, bool AHEAD = true>
+__device__ __forceinline__ double str_single(const VVParams& P, u64 a, u64 b, int spin, W x, W y) {
+    const W d = x ^ y;
+    return single_elem<AHEAD>(P.C, a, b, spin, low_w((W)(x & d)), low_w((W)(y & d)));   // bra -> ket orbital
 }
 
 // Same-spin double: bra string x -> ket string y (differ in 4 bits).
-__device__ __forceinline__ double str_double_same(const VVParams& P, u64 x, u64 y) {
-    const u64 d = x ^ y;
-    u64 pb = x & d, hk = y & d;
-    const int p0 = __ffsll(pb) - 1;
-    pb &= pb - 1;
-    const int p1 = __ffsll(pb) - 1;
-    const int h0 = __ffsll(hk) - 1;
-    hk &= hk - 1;
-    const int h1 = __ffsll(hk) - 1;
+template <class W>
+__device__ __forceinline__ double str_double_same(const VVParams& P, W x, W y) {
+    const W pb = x & ~y, hk = y & ~x;
+    const int p0 = low_w(pb), p1 = high_w(pb), h0 = low_w(hk), h1 = high_w(hk);
     // anti(p0,p1,h0,h1) = (p0 h0|p1 h1) - (p0 h1|p1 h0)   (ham_eval.cpp:124-139)
-    const double raw = eri(P.E, p0, h0, p1, h1) - eri(P.E, p0, h1, p1, h0);
-    int perm = occ_between(x, h0, p0) + occ_between(x, h1, p1);
+    const double raw = eri(P.E, tri2(p0, h0), tri2(p1, h1)) - eri(P.E, tri2(p0, h1), tri2(p1, h0));
+    int perm = between_w(x, h0, p0) + between_w(x, h1, p1);
     const int A = min(h0, p0), B = max(h0, p0), Cc = min(h1, p1), D = max(h1, p1);
     if ((Cc > A && Cc < B && D > B) || (A > Cc && A < D && B > D)) ++perm;
     return (perm & 1) ? -raw : raw;
@@ -752,17 +765,19 @@ __device__ __forceinline__ void load_lists(WarpShared& S, u64 a, u64 b, int n_or
 }
 
 // A connected member of a row is a (sorted position, tag) pair: the tag's
-// low byte is its kind, and for opposite-spin doubles bits 8-15 / 16-23
-// hold the alpha hole and particle.  The diagonal is a member of its own
+// low byte is its kind, and for opposite-spin doubles bits 8-20 hold the
+// excitation of the string whose groups were walked.  The diagonal is a member of its own
 // kind whose position is the row.  Members are found by walk_row and
 // turned into elements by eval_hit, in the order found.
 // kinds: same beta string, same alpha string, opposite-spin double found
 // through the alpha groups (position in the alpha-sorted order, tag with the
-// alpha hole and particle), diagonal, a single evaluated ahead (its position
-// field is its index in the singles list), opposite-spin double found
-// through the beta groups (position in the beta-sorted order, tag with the
-// beta hole and particle).  kSingleBit marks a single of kind A or B as the
-// walk finds it.
+// alpha excitation), diagonal, a single evaluated ahead (its position field
+// is its index in the singles list), opposite-spin double found through the
+// beta groups (position in the beta-sorted order, tag with the beta
+// excitation).  kSingleBit marks a single of kind A or B as the walk finds
+// it.  The excitation of a tag is what the element needs of it: the key of
+// its (hole, particle) pair in bits 8-19 and the parity of the occupied
+// orbitals between them in bit 20, worked out once per group of the walk.
 enum : u32 { kHitA = 0, kHitB = 1, kHitC = 2, kHitD = 3, kHitS = 4, kHitC2 = 5 };
 constexpr u32 kSingleBit = 0x80;
 
@@ -772,60 +787,6 @@ struct Hit {
     bool keep;
 };
 
-__device__ __forceinline__ Hit eval_hit(const VVParams& P, int r, u64 a, u64 b, double psr,
-                                        double cut, u32 pos, u32 tag,
-                                        const SingleOut* sres = nullptr) {
-    Hit e{0.0, 0u, false};
-    const u32 kind = tag & 0x7f;
-    if (kind == kHitS) {
-        const SingleOut o = sres[pos];
-        e.h = o.h;
-        e.j = o.j;
-        e.keep = o.keep != 0;
-    } else if (kind == kHitC) {
-        const u64 y = __ldg(&P.a_other[pos]);
-        const u64 x = b ^ y;
-        const int ha = (tag >> 8) & 0xff, pa = tag >> 16;
-        const int hb = __ffsll(b & x) - 1, pb = __ffsll(y & x) - 1;
-        const double raw = eri(P.E, ha, pa, hb, pb);   // (a i|b j)
-        const int perm = occ_between(a, pa, ha) + occ_between(b, pb, hb);
-        e.h = (perm & 1) ? -raw : raw;
-        e.keep = keep_double(cut, e.h);
-        if (e.keep) e.j = __ldg(&P.a_idx[pos]);
-    } else if (kind == kHitC2) {
-        const u64 y = __ldg(&P.b_other[pos]);   // the member's alpha string
-        const u64 x = a ^ y;
-        const int hb = (tag >> 8) & 0xff, pb = tag >> 16;
-        const int ha = __ffsll(a & x) - 1, pa = __ffsll(y & x) - 1;
-        const double raw = eri(P.E, ha, pa, hb, pb);   // (a i|b j)
-        const int perm = occ_between(a, pa, ha) + occ_between(b, pb, hb);
-        e.h = (perm & 1) ? -raw : raw;
-        e.keep = keep_double(cut, e.h);
-        if (e.keep) e.j = __ldg(&P.b_idx[pos]);
-    } else if (kind == kHitD) {
-        e.h = P.diag[r];
-        e.keep = fabs(e.h) > kElemThresh;
-        e.j = (u32)r;
-    } else {
-        const bool alpha = kind == kHitA;   // the alpha string moves
-        const u64 y = alpha ? __ldg(&P.b_other[pos]) : __ldg(&P.a_other[pos]);
-        const u64 x = alpha ? a : b;
-        if (__popcll(x ^ y) == 2) {
-            e.h = str_single(P, a, b, alpha ? 0 : 1, x, y);
-            e.keep = keep_single(P, psr, e.h);
-        } else {
-            e.h = str_double_same(P, x, y);
-            e.keep = keep_double(cut, e.h);
-        }
-        if (e.keep) e.j = alpha ? __ldg(&P.b_idx[pos]) : __ldg(&P.a_idx[pos]);
-    }
-    return e;
-}
-
-// Scans read the companion strings as W: u32 when every string fits in 32
-// orbitals (half the bytes, one xor and popcount per test), else u64.
-__device__ __forceinline__ int popc_w(u32 x) { return __popc(x); }
-__device__ __forceinline__ int popc_w(u64 x) { return __popcll(x); }
 template <class W> __device__ __forceinline__ const W* a_others(const VVParams& P);
 template <class W> __device__ __forceinline__ const W* b_others(const VVParams& P);
 template <> __device__ __forceinline__ const u64* a_others<u64>(const VVParams& P) {
@@ -841,6 +802,61 @@ template <> __device__ __forceinline__ const u32* b_others<u32>(const VVParams& 
     return P.b_other32;
 }
 
+// Tag of an opposite-spin double through the single h -> p of string x.
+template <class W>
+__device__ __forceinline__ u32 exc_tag(u32 kind, W x, int h, int p) {
+    return kind | tri2(h, p) << 8 | (u32)(between_w(x, h, p) & 1) << 20;
+}
+
+// Bound: instructions and the latency of the gathers (string, index,
+// integral): 327 instructions per 32 members of a 30-orbital space with 64-bit
+// strings, index and phase arithmetic.  k_vv_eval at 1e6 rows 3.80 -> 2.77 ms.
+// AHEAD: singles read their integrals ahead of the additions.
+template <class W, bool AHEAD = true>
+__device__ __forceinline__ Hit eval_hit(const VVParams& P, int r, u64 a, u64 b, double psr,
+                                        double cut, u32 pos, u32 tag,
+                                        const SingleOut* sres = nullptr) {
+    Hit e{0.0, 0u, false};
+    const u32 kind = tag & 0x7f;
+    if (kind == kHitS) {
+        const SingleOut o = sres[pos];
+        e.h = o.h;
+        e.j = o.j;
+        e.keep = o.keep != 0;
+    } else if (kind == kHitC || kind == kHitC2) {
+        // the member's string on the other side differs from the row's in one
+        // pair; (a i|b j) and the phase are symmetric in its two orbitals
+        const bool c2 = kind == kHitC2;
+        const W s = (W)(c2 ? a : b);
+        const W x = s ^ __ldg(&(c2 ? b_others<W>(P) : a_others<W>(P))[pos]);
+        const u32 j = __ldg(&(c2 ? P.b_idx : P.a_idx)[pos]);
+        const int lo = low_w(x), hi = high_w(x);
+        const double raw = eri(P.E, (tag >> 8) & 0xfffu, tri2(hi, lo));
+        const u32 odd = (u32)between_w(s, lo, hi) ^ (tag >> 20);
+        e.h = (odd & 1u) ? -raw : raw;
+        e.keep = keep_double(cut, e.h);
+        e.j = j;
+    } else if (kind == kHitD) {
+        e.h = P.diag[r];
+        e.keep = fabs(e.h) > kElemThresh;
+        e.j = (u32)r;
+    } else {
+        const bool alpha = kind == kHitA;   // the alpha string moves
+        const W y = __ldg(&(alpha ? b_others<W>(P) : a_others<W>(P))[pos]);
+        const W x = (W)(alpha ? a : b);
+        const u32 j = __ldg(&(alpha ? P.b_idx : P.a_idx)[pos]);
+        if (popc_w((W)(x ^ y)) == 2) {
+            e.h = str_single<W, AHEAD>(P, a, b, alpha ? 0 : 1, x, y);
+            e.keep = keep_single(P, psr, e.h);
+        } else {
+            e.h = str_double_same<W>(P, x, y);
+            e.keep = keep_double(cut, e.h);
+        }
+        e.j = j;
+    }
+    return e;
+}
+
 // Part C over the short groups of one round of 32 alpha singles, packed:
 // the members of all of them are numbered in group order and each step
 // tests 32 consecutive members.  The nonempty groups take slots in lane
@@ -850,8 +866,8 @@ template <> __device__ __forceinline__ const u32* b_others<u32>(const VVParams& 
 // covers windows of 32 * kWinW members.
 template <class W, class Q>
 __device__ __forceinline__ void part_c_packed(Q& q, WarpShared& S, const W* a_other, W b,
-                                              unsigned long long& tests, u32 gs, u32 sl, int hh,
-                                              int pp, u32 kind) {
+                                              unsigned long long& tests, u32 gs, u32 sl,
+                                              u32 tag) {
     const int lane = threadIdx.x & 31;
     u32 incl = sl;   // inclusive prefix over lanes
 #pragma unroll
@@ -866,7 +882,7 @@ __device__ __forceinline__ void part_c_packed(Q& q, WarpShared& S, const W* a_ot
         const int slot = __popc(ne & lanemask_lt());
         const u32 pre = incl - sl;   // first member of this lane's group
         S.off[slot] = gs - pre;
-        S.tg[slot] = kind | ((u32)hh << 8) | ((u32)pp << 16);
+        S.tg[slot] = tag;
         S.first[slot] = pre;
     }
     const int ns = __popc(ne);
@@ -1001,12 +1017,11 @@ __device__ __forceinline__ void part_c(const VVParams& P, WarpShared& S, Q& q,
         const u32 gcur = gnext;
         if (nrow != 0xffffffffu && sidx + step < nsx)
             gnext = __ldg(&(bm ? P.b_nbr : P.a_nbr)[nrow + sidx + step]);
-        u32 gs = 0, gl = 0, gg = 0xffffffffu;
-        int hh = 0, pp = 0;
+        u32 gs = 0, gl = 0, gg = 0xffffffffu, mytag = 0;
         if (sidx < nsx) {
             int pi;
-            hh = occx[small_div(sidx, rvx, nvx, pi)];
-            pp = virx[pi];
+            const int hh = occx[small_div(sidx, rvx, nvx, pi)], pp = virx[pi];
+            mytag = exc_tag(kind, (W)x, hh, pp);
             if (nrow != 0xffffffffu) {
                 gg = gcur;
                 if (gg != 0xffffffffu) {
@@ -1029,7 +1044,7 @@ __device__ __forceinline__ void part_c(const VVParams& P, WarpShared& S, Q& q,
                                                           : __ldg(&(bm ? P.b_gid : P.a_gid)[gs])])
                  : 0u;
         if (!P.c_groupwalk) {
-            part_c_packed(q, S, xo, yw, tests, gs, small ? gl : 0u, hh, pp, kind);
+            part_c_packed(q, S, xo, yw, tests, gs, small ? gl : 0u, mytag);
         } else {
             // one group at a time: start, length and the x excitation are
             // warp-uniform, members in order 32 per step
@@ -1039,8 +1054,7 @@ __device__ __forceinline__ void part_c(const VVParams& P, WarpShared& S, Q& q,
                 m &= m - 1;
                 const u32 g0 = __shfl_sync(0xffffffffu, gs, L);
                 const u32 gn = __shfl_sync(0xffffffffu, gl, L);
-                const u32 tag = kind | ((u32)__shfl_sync(0xffffffffu, hh, L) << 8) |
-                                ((u32)__shfl_sync(0xffffffffu, pp, L) << 16);
+                const u32 tag = __shfl_sync(0xffffffffu, mytag, L);
                 tests += gn;
                 for (u32 t0 = 0; t0 < gn; t0 += 32 * kScanU) {
                     W w[kScanU];
@@ -1099,8 +1113,7 @@ __device__ __forceinline__ void part_c(const VVParams& P, WarpShared& S, Q& q,
             const int L = __ffs(pm) - 1;
             pm &= pm - 1;
             const u32 g0 = __shfl_sync(0xffffffffu, gs, L);
-            const u32 tag = kind | ((u32)__shfl_sync(0xffffffffu, hh, L) << 8) |
-                            ((u32)__shfl_sync(0xffffffffu, pp, L) << 16);
+            const u32 tag = __shfl_sync(0xffffffffu, mytag, L);
             const uint2* row =
                 pres + (i64)__shfl_sync(0xffffffffu, prw, L) * (bm ? P.pres_words_b : P.pres_words);
             tests += nys;
@@ -1134,8 +1147,7 @@ __device__ __forceinline__ void part_c(const VVParams& P, WarpShared& S, Q& q,
             bigm &= bigm - 1;
             const u32 g0 = __shfl_sync(0xffffffffu, gs, L);
             const u32 gn = __shfl_sync(0xffffffffu, gl, L);
-            const u32 tag = kind | ((u32)__shfl_sync(0xffffffffu, hh, L) << 8) |
-                            ((u32)__shfl_sync(0xffffffffu, pp, L) << 16);
+            const u32 tag = __shfl_sync(0xffffffffu, mytag, L);
             tests += nyv;
             for (int q0 = 0; q0 < nyv; q0 += 32) {
                 const int qi = q0 + lane;
@@ -1296,7 +1308,7 @@ struct HitOut {
 
 // Sink of walk_row that evaluates as it goes (the long-row and two-pass
 // walks): members queue in shared memory and are evaluated 32 at a time.
-template <class Out>
+template <class Out, class W>
 struct QueueEval {
     const VVParams& P;
     int r;
@@ -1323,7 +1335,7 @@ struct QueueEval {
         if (lane < cnt) {
             int k = head + lane;
             if (k >= kRing) k -= kRing;
-            e = eval_hit(P, r, a, b, psr, cut, Q.pos[k], Q.tag[k]);
+            e = eval_hit<W, false>(P, r, a, b, psr, cut, Q.pos[k], Q.tag[k]);
         }
         out.put(e.keep, e.j, e.h);
         head += cnt;
@@ -1353,7 +1365,7 @@ struct QueueEval {
 template <class Out>
 __device__ void vv_row(const VVParams& P, int r, u64 a, u64 b, double psr, double cut,
                        WarpShared& S, HitRing& ring, Out& out, unsigned long long& tests) {
-    QueueEval<Out> q{P, r, a, b, psr, cut, ring, out};
+    QueueEval<Out, u64> q{P, r, a, b, psr, cut, ring, out};
     walk_row<u64>(P, r, a, b, S, q, tests);
     q.flush();
 }
@@ -1511,7 +1523,7 @@ __global__ void __launch_bounds__(256) k_vv_singles(Loc L, Arena A) {
         row_setup(P, r, a, b, psr, cut);
         const bool alpha = e.z == kHitA;   // the alpha string moves
         const u64 y = alpha ? __ldg(&P.b_other[e.y]) : __ldg(&P.a_other[e.y]);
-        const double h = str_single(P, a, b, alpha ? 0 : 1, alpha ? a : b, y);
+        const double h = str_single<u64>(P, a, b, alpha ? 0 : 1, alpha ? a : b, y);
         SingleOut o;
         o.h = h;
         o.keep = keep_single(P, psr, h) ? 1u : 0u;
@@ -1528,7 +1540,17 @@ __global__ void __launch_bounds__(256) k_vv_singles(Loc L, Arena A) {
 // connected to most of a small space took 60 of 67 us at 2,241 rows): it
 // joins the rows that k_vv_eval_long spreads over the grid.
 constexpr unsigned long long kLongEval = 512;
-template <class Loc>
+template <class W>
+__device__ __forceinline__ Hit eval_any(const VVParams& P, int r, u64 a, u64 b, double psr,
+                                        double cut, u32 pos, u32 tag, const SingleOut* sres) {
+    if constexpr (std::is_same<W, PerRowW>::value) {
+        return P.a_other32 ? eval_hit<u32>(P, r, a, b, psr, cut, pos, tag, sres)
+                           : eval_hit<u64>(P, r, a, b, psr, cut, pos, tag, sres);
+    } else {
+        return eval_hit<W>(P, r, a, b, psr, cut, pos, tag, sres);
+    }
+}
+template <class Loc, class W>
 __global__ void __launch_bounds__(kWS * 32) k_vv_eval(Loc L, Arena A) {
     const int lane = threadIdx.x & 31;
     const i64 gw = (blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5;
@@ -1559,8 +1581,8 @@ __global__ void __launch_bounds__(kWS * 32) k_vv_eval(Loc L, Arena A) {
             const u64 m2 = k2 < len ? mem[pos + k2] : 0ull;
             const u32 p1 = (u32)m1, t1 = (u32)(m1 >> 32), p2 = (u32)m2, t2 = (u32)(m2 >> 32);
             Hit e1{0.0, 0u, false}, e2{0.0, 0u, false};
-            if (k1 < len) e1 = eval_hit(P, r, a, b, psr, cut, p1, t1, A.sres);
-            if (k2 < len) e2 = eval_hit(P, r, a, b, psr, cut, p2, t2, A.sres);
+            if (k1 < len) e1 = eval_any<W>(P, r, a, b, psr, cut, p1, t1, A.sres);
+            if (k2 < len) e2 = eval_any<W>(P, r, a, b, psr, cut, p2, t2, A.sres);
             unsigned m = __ballot_sync(0xffffffffu, e1.keep);
             if (e1.keep) {
                 const i64 at = w + __popc(m & lanemask_lt());
@@ -1644,7 +1666,7 @@ inline i64 unit_bound(i64 slots, i64 nrows) { return slots / 64 + nrows + 1; }
 // The members of the long rows become entries in place, a 64-member unit per
 // warp step over the whole grid; a dropped member leaves a hole.  Kept counts
 // are summed into row_len.
-template <class Loc>
+template <class Loc, class W>
 __global__ void __launch_bounds__(kWS * 32) k_vv_eval_long(Loc L, Arena A) {
     const int lane = threadIdx.x & 31;
     const i64 gw = (blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5;
@@ -1670,7 +1692,8 @@ __global__ void __launch_bounds__(kWS * 32) k_vv_eval_long(Loc L, Arena A) {
             bool keep = false;
             if (k < len) {
                 const u64 m = mem[pos + k];
-                const Hit e = eval_hit(P, r, a, b, psr, cut, (u32)m, (u32)(m >> 32), A.sres);
+                const Hit e =
+                    eval_any<W>(P, r, a, b, psr, cut, (u32)m, (u32)(m >> 32), A.sres);
                 keep = e.keep;
                 A.acol[pos + k] = e.keep ? e.j + cb : kHole;
                 A.aval[pos + k] = e.h;
@@ -1993,15 +2016,6 @@ void build_row_order(const StrIndex& A, const StrIndex& B, const u64* V, i64 n, 
     DNQ_CHECK_LAUNCH();
 }
 
-// Grid of k_vv_eval: as many blocks as fit (it holds fewer registers than
-// the walk, and more warps in flight hide more of its gather latency).
-template <class Loc>
-int eval_grid(int device) {
-    int per_sm = 0;
-    DNQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_vv_eval<Loc>, kWS * 32, 0));
-    return std::max(1, per_sm) * sm_count(device);
-}
-
 // scan: 0 = 64-bit strings, 1 = 32-bit, 2 = chosen per row.
 template <class Loc>
 void launch_walk(int scan, int grid, const Loc& L, const Arena& A, cudaStream_t s) {
@@ -2016,6 +2030,29 @@ void launch_big(int scan, int grid, const Loc& L, const Arena& A, cudaStream_t s
     if (scan == 1) k_vv_big<Loc, u32><<<grid, kWS * 32, 0, s>>>(L, A);
     else if (scan == 2) k_vv_big<Loc, PerRowW><<<grid, kWS * 32, 0, s>>>(L, A);
     else k_vv_big<Loc, u64><<<grid, kWS * 32, 0, s>>>(L, A);
+    DNQ_CHECK_LAUNCH();
+}
+
+// k_vv_eval on as many blocks as fit (it holds fewer registers than the walk,
+// and more warps in flight hide more of its gather latency).
+template <class Loc>
+void launch_eval(int scan, int device, const Loc& L, const Arena& A, cudaStream_t s) {
+    auto go = [&](auto kern) {
+        int per_sm = 0;
+        DNQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWS * 32, 0));
+        kern<<<std::max(1, per_sm) * sm_count(device), kWS * 32, 0, s>>>(L, A);
+    };
+    if (scan == 1) go(k_vv_eval<Loc, u32>);
+    else if (scan == 2) go(k_vv_eval<Loc, PerRowW>);
+    else go(k_vv_eval<Loc, u64>);
+    DNQ_CHECK_LAUNCH();
+}
+
+template <class Loc>
+void launch_eval_long(int scan, int grid, const Loc& L, const Arena& A, cudaStream_t s) {
+    if (scan == 1) k_vv_eval_long<Loc, u32><<<grid, kWS * 32, 0, s>>>(L, A);
+    else if (scan == 2) k_vv_eval_long<Loc, PerRowW><<<grid, kWS * 32, 0, s>>>(L, A);
+    else k_vv_eval_long<Loc, u64><<<grid, kWS * 32, 0, s>>>(L, A);
     DNQ_CHECK_LAUNCH();
 }
 
@@ -2112,12 +2149,9 @@ i64 run_vv(const Loc& L, i64 nrows, i64 cap_hint, int device, cudaStream_t s, Cs
     launch_walk<Loc>(scan, grid, L, A, s);
     k_vv_singles<Loc><<<grid, 256, 0, s>>>(L, A);
     DNQ_CHECK_LAUNCH();
-    k_vv_eval<Loc><<<eval_grid<Loc>(device), kWS * 32, 0, s>>>(L, A);
-    DNQ_CHECK_LAUNCH();
+    launch_eval<Loc>(scan, device, L, A, s);
     launch_big<Loc>(scan, grid, L, A, s);
-    DNQ_CHECK_LAUNCH();
-    k_vv_eval_long<Loc><<<grid, kWS * 32, 0, s>>>(L, A);
-    DNQ_CHECK_LAUNCH();
+    launch_eval_long<Loc>(scan, grid, L, A, s);
     int hov = 0;
     unsigned long long hcur = 0;   // arena slots handed out (chunks and long rows)
     DNQ_CUDA(cudaMemcpyAsync(&hov, ovf.p, 4, cudaMemcpyDeviceToHost, s));
@@ -2656,7 +2690,7 @@ k_contract_walk(VVParams P, const double* coeff, const uint2* item, i64 n_item, 
         row_setup(P, r, a, b, psr, cut);
         load_lists(S, a, b, P.n_orb);
         ContractOut out{coeff};
-        QueueEval<ContractOut> q{P, r, a, b, psr, cut, R, out};
+        QueueEval<ContractOut, W> q{P, r, a, b, psr, cut, R, out};
         unsigned long long tests = 0;
         walk_row<W, true>(P, r, a, b, S, q, tests, (int)(it.y >> 16), (int)(it.y & 0xffffu));
         q.flush();
@@ -2984,11 +3018,9 @@ void enqueue_step(dnq_batch_s* b, int precision, cudaStream_t s, cudaEvent_t* ev
     launch_walk<ManySys>(b->scan, grid, L, A, s);
     k_vv_singles<ManySys><<<grid, 256, 0, s>>>(L, A);
     DNQ_CHECK_LAUNCH();
-    k_vv_eval<ManySys><<<eval_grid<ManySys>(b->device), kWS * 32, 0, s>>>(L, A);
-    DNQ_CHECK_LAUNCH();
+    launch_eval<ManySys>(b->scan, b->device, L, A, s);
     launch_big<ManySys>(b->scan, grid, L, A, s);
-    k_vv_eval_long<ManySys><<<grid, kWS * 32, 0, s>>>(L, A);
-    DNQ_CHECK_LAUNCH();
+    launch_eval_long<ManySys>(b->scan, grid, L, A, s);
     mark(2);
     prim::scan<u32, i64, false>(b->rlen.p, b->M.rowptr.p, n + 1, s, b->scan_tmp.p);
     k_sanitize<<<1, 1024, 0, s>>>(b->M.rowptr.p, n, b->M.nnz, b->ovf.p, b->bad.p);
