@@ -71,11 +71,12 @@ struct BuildParams {
     i64 nV;
     const double* diag;
     int* next_row;
-    // count pass
+    int parts;             // units of work per row (enumerate_row)
+    // count pass, per unit
     u32* cnt_vv;
     u32* cnt_vp;
     unsigned long long* n_cand;
-    // fill pass
+    // fill pass, per unit
     const i64* off_vv;
     const i64* off_vp;
     u32* vv_col;
@@ -147,10 +148,11 @@ k_build(BuildParams P) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WarpRow& R = rows[w];
     for (;;) {
-        int r = 0;
-        if (lane == 0) r = atomicAdd(P.next_row, 1);
-        r = __shfl_sync(0xffffffffu, r, 0);
-        if (r >= P.nV) break;
+        int unit = 0;
+        if (lane == 0) unit = atomicAdd(P.next_row, 1);
+        unit = __shfl_sync(0xffffffffu, unit, 0);
+        if (unit >= P.nV * P.parts) break;
+        const int r = unit / P.parts, part = unit % P.parts;
         load_row(R, P.V[2 * (i64)r], P.V[2 * (i64)r + 1], P.n_orb);
         double psr = 0.0, cut = P.cut;
         if (P.policy == DNQ_POLICY_DYNAMIC) {
@@ -161,10 +163,10 @@ k_build(BuildParams P) {
         }
         BuildSink<FILL> sink(P, psr);
         const double d = P.diag[r];
-        const bool dkeep = fabs(d) > kElemThresh;
+        const bool dkeep = part == 0 && fabs(d) > kElemThresh;
         if (FILL) {
-            sink.wvv = P.off_vv[r];
-            sink.wvp = P.off_vp[r];
+            sink.wvv = P.off_vv[unit];
+            sink.wvp = P.off_vp[unit];
             if (dkeep) {
                 if (lane == 0) {
                     P.vv_col[sink.wvv] = (u32)r;
@@ -175,15 +177,16 @@ k_build(BuildParams P) {
         } else if (dkeep && lane == 0) {
             sink.nvv = 1;
         }
-        enumerate_row(P.C, R, P.policy == DNQ_POLICY_DYNAMIC ? nullptr : P.plen, cut, sink);
+        enumerate_row(P.C, R, P.policy == DNQ_POLICY_DYNAMIC ? nullptr : P.plen, cut, sink, part,
+                      P.parts);
         if (!FILL) {
             const u32 a = __reduce_add_sync(0xffffffffu, sink.nvv);
             const u32 b = __reduce_add_sync(0xffffffffu, sink.nvp);
             unsigned long long c = sink.ncand;
             for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
             if (lane == 0) {
-                P.cnt_vv[r] = a;
-                P.cnt_vp[r] = b;
+                P.cnt_vv[unit] = a;
+                P.cnt_vp[unit] = b;
                 atomicAdd(P.n_cand, c);
             }
         }
@@ -238,29 +241,44 @@ __global__ void k_val_f32_tail(const double* v, i64 n, float* o) {
 }
 
 // Diagonal entry of each row (column order not assumed): moved out of the
-// FP32 copy into the FP64 vector (0 when the row has none).  Warp per row.
+// FP32 copy into the FP64 vector (0 when the row has none).  A lane looks at
+// its row's first entry, where the V->V build puts the diagonal; the rows
+// whose diagonal is elsewhere are searched by the warp one after the other.
+// (A warp per row spent 160 us on the latency of 1e6 first entries.)
 __global__ void k_split_diag(const i64* rs, const i64* re, const u32* col, const double* val,
                              i64 nr, float* out, double* dout) {
     const int lane = threadIdx.x & 31;
     const i64 gw = (blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5;
     const i64 nw = (gridDim.x * (i64)blockDim.x) >> 5;
-    for (i64 r = gw; r < nr; r += nw) {
-        const i64 b = rs[r], e = re[r];
-        double d = 0.0;
-        for (i64 k0 = b; k0 < e; k0 += 32) {
-            const i64 k = k0 + lane;
-            const bool on = k < e && col[k] == (u32)r;
-            if (on) {
-                d = val[k];
-                out[k] = 0.0f;
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, on);
-            if (m) {
-                d = __shfl_sync(0xffffffffu, d, __ffs(m) - 1);
-                break;
-            }
+    for (i64 r0 = 32 * gw; r0 < nr; r0 += 32 * nw) {
+        const i64 mine = r0 + lane;
+        const i64 mb = mine < nr ? rs[mine] : 0, me = mine < nr ? re[mine] : 0;
+        const bool first = mb < me && col[mb] == (u32)mine;
+        if (first) {
+            if (dout) dout[mine] = val[mb];
+            out[mb] = 0.0f;
         }
-        if (dout && lane == 0) dout[r] = d;
+        for (unsigned todo = __ballot_sync(0xffffffffu, !first && mine < nr); todo;
+             todo &= todo - 1) {
+            const int src = __ffs(todo) - 1;
+            const i64 r = r0 + src;
+            const i64 b = __shfl_sync(0xffffffffu, mb, src), e = __shfl_sync(0xffffffffu, me, src);
+            double d = 0.0;
+            for (i64 k0 = b; k0 < e; k0 += 32) {
+                const i64 k = k0 + lane;
+                const bool on = k < e && col[k] == (u32)r;
+                if (on) {
+                    d = val[k];
+                    out[k] = 0.0f;
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, on);
+                if (m) {
+                    d = __shfl_sync(0xffffffffu, d, __ffs(m) - 1);
+                    break;
+                }
+            }
+            if (dout && lane == 0) dout[r] = d;
+        }
     }
 }
 
@@ -274,13 +292,6 @@ inline int grid_for(i64 n, int threads = 256) {
 template <class T>
 void exclusive_scan(const T* in, i64* out, i64 n, cudaStream_t s) {
     prim::scan<T, i64, false>(in, out, n, s);
-}
-
-i64 read_i64(const i64* d, cudaStream_t s) {
-    i64 v = 0;
-    DNQ_CUDA(cudaMemcpyAsync(&v, d, sizeof(i64), cudaMemcpyDeviceToHost, s));
-    DNQ_CUDA(cudaStreamSynchronize(s));
-    return v;
 }
 
 }  // namespace
@@ -322,7 +333,7 @@ void launch_f32_split(const Csr& m, float* val32, double* diag_out, cudaStream_t
 }
 
 void make_f32(Csr& m, cudaStream_t s, DBuf<double>* diag_out) {
-    m.val32.alloc(m.val.n, s);
+    m.val32.alloc(m.span(), s);
     if (diag_out) diag_out->alloc(m.nr, s);
     if (m.nr == 0) return;
     launch_f32_split(m, m.val32.p, diag_out ? diag_out->p : nullptr, s);
@@ -473,22 +484,24 @@ void build_ham(dnq_ctx_s* ctx, const u64* V_in, i64 nV, const u64* X_in, i64 nX,
         DNQ_CHECK_LAUNCH();
         P.plen = plen.p;
     }
+    int dev_sms = sm_count(ctx->device);
+    int per_sm = 0;
+    DNQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_build<false>,
+                                                           kWarpsPerBlock * 32, 0));
+    const int grid = std::max(1, per_sm) * dev_sms;
+    P.parts = row_parts(nV, (i64)grid * kWarpsPerBlock, n_orb);
+    const i64 nu = nV * P.parts;   // units of work
     DBuf<int> next(1, s);
-    DBuf<u32> cvv(nV + 1, s), cvp(nV + 1, s);
+    DBuf<u32> cvv(nu + 1, s), cvp(nu + 1, s);
     DBuf<unsigned long long> ncand(1, s);
-    DNQ_CUDA(cudaMemsetAsync(cvv.p + nV, 0, 4, s));
-    DNQ_CUDA(cudaMemsetAsync(cvp.p + nV, 0, 4, s));
+    DNQ_CUDA(cudaMemsetAsync(cvv.p + nu, 0, 4, s));
+    DNQ_CUDA(cudaMemsetAsync(cvp.p + nu, 0, 4, s));
     DNQ_CUDA(cudaMemsetAsync(ncand.p, 0, 8, s));
     P.next_row = next.p;
     P.cnt_vv = cvv.p;
     P.cnt_vp = cvp.p;
     P.n_cand = ncand.p;
 
-    int dev_sms = sm_count(ctx->device);
-    int per_sm = 0;
-    DNQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_build<false>,
-                                                           kWarpsPerBlock * 32, 0));
-    const int grid = std::max(1, per_sm) * dev_sms;
     DNQ_CUDA(cudaMemsetAsync(next.p, 0, 4, s));
     T.mark();
     k_build<false><<<grid, kWarpsPerBlock * 32, 0, s>>>(P);
@@ -497,13 +510,14 @@ void build_ham(dnq_ctx_s* ctx, const u64* V_in, i64 nV, const u64* X_in, i64 nX,
 
     H->vv.nr = nV;
     H->vv.nc = nV;
-    H->vv.rowptr.alloc(nV + 1, s);
-    exclusive_scan(cvv.p, H->vv.rowptr.p, nV + 1, s);
-    DBuf<i64> offp(nV + 1, s);
-    exclusive_scan(cvp.p, offp.p, nV + 1, s);
-    H->vv.nnz = read_i64(H->vv.rowptr.p + nV, s);
-    const i64 nvp = read_i64(offp.p + nV, s);
+    DBuf<i64> uvv(nu + 1, s), uvp(nu + 1, s);
+    exclusive_scan(cvv.p, uvv.p, nu + 1, s);
+    exclusive_scan(cvp.p, uvp.p, nu + 1, s);
+    i64 nvp = 0;
+    DNQ_CUDA(cudaMemcpyAsync(&H->vv.nnz, uvv.p + nu, 8, cudaMemcpyDeviceToHost, s));
+    DNQ_CUDA(cudaMemcpyAsync(&nvp, uvp.p + nu, 8, cudaMemcpyDeviceToHost, s));
     DNQ_CUDA(cudaMemcpyAsync(&H->candidates, ncand.p, 8, cudaMemcpyDeviceToHost, s));
+    DNQ_CUDA(cudaStreamSynchronize(s));
 
     H->vv.col.alloc(H->vv.nnz, s);
     H->vv.val.alloc(H->vv.nnz, s);
@@ -512,8 +526,8 @@ void build_ham(dnq_ctx_s* ctx, const u64* V_in, i64 nV, const u64* X_in, i64 nX,
     DBuf<double> vp_val(nvp, s);
     if (has_ext) vp_col.alloc(nvp, s);
     else vp_key.alloc(nvp, s);
-    P.off_vv = H->vv.rowptr.p;
-    P.off_vp = offp.p;
+    P.off_vv = uvv.p;
+    P.off_vp = uvp.p;
     P.vv_col = H->vv.col.p;
     P.vv_val = H->vv.val.p;
     P.vp_col = vp_col.p;
@@ -524,6 +538,18 @@ void build_ham(dnq_ctx_s* ctx, const u64* V_in, i64 nV, const u64* X_in, i64 nX,
     k_build<true><<<grid, kWarpsPerBlock * 32, 0, s>>>(P);
     DNQ_CHECK_LAUNCH();
     T.mark();
+    DBuf<i64> offp;
+    if (P.parts == 1) {
+        H->vv.rowptr = std::move(uvv);
+        offp = std::move(uvp);
+    } else {
+        H->vv.rowptr.alloc(nV + 1, s);
+        offp.alloc(nV + 1, s);
+        k_first_parts<<<grid_for(nV + 1), 256, 0, s>>>(uvv.p, P.parts, nV, H->vv.rowptr.p);
+        DNQ_CHECK_LAUNCH();
+        k_first_parts<<<grid_for(nV + 1), 256, 0, s>>>(uvp.p, P.parts, nV, offp.p);
+        DNQ_CHECK_LAUNCH();
+    }
     sort_rows(H->vv, s);
     T.mark();
 

@@ -298,6 +298,16 @@ void order_ties_for(dnq_ctx_s* c, double thr) {
     T.tie_threshold = thr;
 }
 
+// t[h][k][p] = x[h][p][k].
+__global__ void k_swap_last(const double* x, int n, double* t) {
+    const i64 nn = (i64)n * n, all = nn * n;
+    for (i64 at = blockIdx.x * (i64)blockDim.x + threadIdx.x; at < all;
+         at += (i64)gridDim.x * blockDim.x) {
+        const i64 h = at / nn, k = at % nn / n, p = at % n;
+        t[at] = x[(h * n + p) * n + k];
+    }
+}
+
 void upload_tables(dnq_ctx_s* c) {
     const int n = c->n;
     const double* E = c->erip.data();
@@ -328,6 +338,11 @@ void upload_tables(dnq_ctx_s* c) {
     up(c->dos, dos);
     up(c->sss, sss);
     up(c->sos, sos);
+    for (auto [x, t] : {std::pair{&c->sss, &c->sssT}, std::pair{&c->sos, &c->sosT}}) {
+        t->alloc(x->n, s);
+        k_swap_last<<<256, 256, 0, s>>>(x->p, n, t->p);
+        DNQ_CHECK_LAUNCH();
+    }
     up(c->erid, c->erip);
     DNQ_CUDA(cudaStreamSynchronize(s));
 }

@@ -9,6 +9,9 @@
 //   dos  [n*n]     (pp|qq)              opposite-spin diagonal pair term
 //   sss  [n*n*n]   (hp|kk) - (hk|kp)    same-spin term of a single h->p
 //   sos  [n*n*n]   (hp|kk)              opposite-spin term of a single h->p
+//   sssT, sosT     the same as [h][k][p]: a warp that evaluates the singles of
+//                  one determinant takes neighbouring p in its lanes and one k
+//                  at a time, so its reads run along p
 //   pair table     for every occupied spin-orbital pair {i>j}: entries
 //                  (a>b, v = <ij||ab>) sorted by |v| descending
 //
@@ -43,6 +46,8 @@ struct CtxView {
     const double* dos = nullptr;
     const double* sss = nullptr;
     const double* sos = nullptr;
+    const double* sssT = nullptr;
+    const double* sosT = nullptr;
     const double* eri = nullptr;   // packed 8-fold (pq|rs), integral_mo.hpp:40-49
     PairTableView tab;
 };
@@ -88,7 +93,7 @@ struct dnq_ctx_s {
     int nso = 0;
     double e_nuc = 0.0;
     std::vector<double> h1p, erip;   // packed host copies
-    dnq::DBuf<double> h1, dss, dos, sss, sos, erid;
+    dnq::DBuf<double> h1, dss, dos, sss, sos, sssT, sosT, erid;
     dnq::PairTable tab;
     bool has_hb = false;
     double hb_thr = 0.0;
@@ -103,6 +108,8 @@ struct dnq_ctx_s {
         c.dos = dos.p;
         c.sss = sss.p;
         c.sos = sos.p;
+        c.sssT = sssT.p;
+        c.sosT = sosT.p;
         c.eri = erid.p;
         c.tab.off = tab.off.p;
         c.tab.ab = tab.ab.p;
@@ -111,7 +118,7 @@ struct dnq_ctx_s {
     }
     int64_t bytes() const {
         return (int64_t)(h1.bytes() + dss.bytes() + dos.bytes() + sss.bytes() +
-                         sos.bytes() + erid.bytes() + tab.bytes());
+                         sos.bytes() + sssT.bytes() + sosT.bytes() + erid.bytes() + tab.bytes());
     }
 };
 

@@ -16,6 +16,8 @@
 // so it can compact survivors with __ballot_sync in candidate order.
 #pragma once
 
+#include <algorithm>
+
 #include "context.cuh"
 #include "detmap.cuh"
 
@@ -29,26 +31,36 @@ struct WarpRow {
     u8 occa[64], occb[64], vira[64], virb[64];
 };
 
+// One lane per orbital: an orbital's place in its list is the count of the
+// listed orbitals below it.
 __device__ __forceinline__ void load_row(WarpRow& R, u64 a, u64 b, int n_orb) {
     const int lane = threadIdx.x & 31;
     const u64 all = low_mask(n_orb);
+    const int na = __popcll(a), nb = __popcll(b);
+    for (int o = lane; o < 64; o += 32) {
+        const u64 below = (1ull << o) - 1ull;
+        const int oa = __popcll(a & below), ob = __popcll(b & below);
+        if ((a >> o) & 1ull) {
+            R.occa[oa] = (u8)o;
+            R.occ[oa] = (u8)(2 * o);
+        } else if (o < n_orb) {
+            R.vira[o - oa] = (u8)o;
+        }
+        if ((b >> o) & 1ull) {
+            R.occb[ob] = (u8)o;
+            R.occ[na + ob] = (u8)(2 * o + 1);
+        } else if (o < n_orb) {
+            R.virb[o - ob] = (u8)o;
+        }
+    }
     if (lane == 0) {
         R.a = a;
         R.b = b;
-        int k = 0, t;
-        t = 0;
-        for (u64 x = a; x; x &= x - 1) { const int o = __ffsll(x) - 1; R.occa[t++] = o; R.occ[k++] = 2 * o; }
-        R.na = t;
-        t = 0;
-        for (u64 x = b; x; x &= x - 1) { const int o = __ffsll(x) - 1; R.occb[t++] = o; R.occ[k++] = 2 * o + 1; }
-        R.nb = t;
-        R.ne = k;
-        t = 0;
-        for (u64 x = ~a & all; x; x &= x - 1) R.vira[t++] = __ffsll(x) - 1;
-        R.nva = t;
-        t = 0;
-        for (u64 x = ~b & all; x; x &= x - 1) R.virb[t++] = __ffsll(x) - 1;
-        R.nvb = t;
+        R.na = na;
+        R.nb = nb;
+        R.ne = na + nb;
+        R.nva = __popcll(~a & all);
+        R.nvb = __popcll(~b & all);
     }
     __syncwarp();
 }
@@ -132,6 +144,45 @@ __device__ __forceinline__ double single_elem(const CtxView& C, u64 a, u64 b, in
     return (perm & 1) ? -e : e;
 }
 
+// e + col[k * n] for the listed occupied orbitals k but `skip`, in order; four
+// reads ahead of their additions.
+__device__ __forceinline__ double add_col(double e, const double* col, int n, const u8* occ,
+                                          int cnt, int skip) {
+    int t = 0;
+    for (; t + 4 <= cnt; t += 4) {
+        double v[4];
+        int o[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            o[q] = occ[t + q];
+            v[q] = __ldg(&col[o[q] * n]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (o[q] != skip) e += v[q];
+    }
+    for (; t < cnt; ++t)
+        if (occ[t] != skip) e += __ldg(&col[occ[t] * n]);
+    return e;
+}
+
+// Unsigned single h -> p in spin s, for warps that evaluate the singles of
+// one determinant from its occupied lists (ham_eval.cpp:88-115: h1, then
+// alpha ascending, then beta ascending).  Lanes hold neighbouring p and share
+// k, so a read of the [h][k][p] tables is a few sectors a warp; from the
+// [h][p][k] tables each lane draws a line of its own, and the L1 serves one
+// line a clock: the count pass of the two-word build (3.2e7 singles of 40
+// terms) took 4.52 ms so, 3.15 from these, and 1.58 with the pairs looked up 32
+// at a time (enumerate_pairs).
+__device__ __forceinline__ double single_sum(const CtxView& C, const u8* occa, int na,
+                                             const u8* occb, int nb, int s, int h, int p) {
+    const int n = C.n;
+    const size_t base = (size_t)h * n * n + p;
+    double e = C.h1[h * n + p];
+    e = add_col(e, (s ? C.sosT : C.sssT) + base, n, occa, na, s ? -1 : h);
+    return add_col(e, (s ? C.sssT : C.sosT) + base, n, occb, nb, s ? h : -1);
+}
+
 // Double i,j -> a,b (spin-orbitals, i > j, a > b) of the bra from the
 // signed table value v = <ij||ab>.
 __device__ __forceinline__ double double_elem(u64 ba, u64 bb, int i, int j, int a, int b,
@@ -154,29 +205,6 @@ __device__ __forceinline__ double double_elem(u64 ba, u64 bb, int i, int j, int 
         perm = occ_between(ba, ha, pa) + occ_between(bb, hb, pb);
     }
     return (perm & 1) ? -raw : raw;
-}
-
-// Length of the prefix of a table row whose weights are >= cut
-// (HeatBathTable::RowView::with_cutoff, hb_table.hpp:131-146), found by the
-// warp with 32-way probing; cut <= 0 keeps the whole row.
-__device__ __forceinline__ i64 warp_prefix(const double* v, i64 len, double cut) {
-    if (cut <= 0.0 || len == 0) return len;
-    const int lane = threadIdx.x & 31;
-    i64 lo = 0, hi = len;   // answer in [lo, hi]
-    while (hi - lo > 32) {
-        const i64 step = (hi - lo + 31) / 32;
-        const i64 x = lo + lane * step;
-        const bool ok = x < hi && fabs(v[x]) >= cut;
-        const int k = __popc(__ballot_sync(0xffffffffu, ok));
-        if (k == 0) return lo;
-        const i64 nlo = lo + (i64)(k - 1) * step + 1;
-        const i64 nhi = min(hi, lo + (i64)k * step);
-        lo = nlo;
-        hi = nhi;
-    }
-    const i64 x = lo + lane;
-    const bool ok = x < hi && fabs(v[x]) >= cut;
-    return lo + __popc(__ballot_sync(0xffffffffu, ok));
 }
 
 // Candidate handed to a sink (per lane).
@@ -221,31 +249,70 @@ __device__ __forceinline__ void enumerate_singles(const CtxView& C, const WarpRo
                 p = R.virb[u % R.nvb];
                 c.b = R.b ^ (1ull << h) ^ (1ull << p);
             }
-            c.h = single_elem(C, R.a, R.b, s, h, p);
+            const double e = single_sum(C, R.occa, R.na, R.occb, R.nb, s, h, p);
+            c.h = (occ_between(s ? R.b : R.a, h, p) & 1) ? -e : e;
         }
         sink.step(c);
     }
 }
 
+// Pair p = x (x - 1) / 2 + y of the occupied list, y < x.
+__device__ __forceinline__ void pair_of(int p, int& x, int& y) {
+    x = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)p)) * 0.5f);
+    while (x * (x - 1) / 2 > p) --x;
+    while ((x + 1) * x / 2 <= p) ++x;
+    y = p - x * (x - 1) / 2;
+}
+
+// Doubles over the occupied pairs [p_lo, p_hi) (x ascending, y < x ascending).
+// The table rows of 32 pairs are looked up at once, a pair per lane, and the
+// prefixes of a cut of the row's own searched side by side: one pair after
+// the other, a warp waits several L2 reads for each, most of them for an empty
+// prefix under dynamic screening.
 template <class Sink>
-__device__ __forceinline__ void enumerate_row(const CtxView& C, const WarpRow& R,
-                                              const i64* plen, double cut, Sink& sink) {
+__device__ __forceinline__ void enumerate_pairs(const CtxView& C, const WarpRow& R,
+                                                const i64* plen, double cut, Sink& sink, int p_lo,
+                                                int p_hi) {
     const int lane = threadIdx.x & 31;
-    enumerate_singles(C, R, sink);
-    // ---- doubles
-    for (int x = 1; x < R.ne; ++x) {
-        const int i = R.occ[x];
-        for (int y = 0; y < x; ++y) {
-            const int j = R.occ[y];
+    for (int p0 = p_lo; p0 < p_hi; p0 += 32) {
+        i64 lo_l = 0;
+        u32 len_l = 0, ij_l = 0;
+        if (p0 + lane < p_hi) {
+            int x, y;
+            pair_of(p0 + lane, x, y);
+            const int i = R.occ[x], j = R.occ[y];
             const i64 row = pair_row(i, j);
-            const i64 lo = __ldg(&C.tab.off[row]);
-            i64 len;
-            if (plen) len = __ldg(&plen[row]);
-            else len = warp_prefix(C.tab.v + lo, __ldg(&C.tab.off[row + 1]) - lo, cut);
-            const int ii = max(i, j), jj = min(i, j);
-            for (i64 e0 = 0; e0 < len; e0 += 32) {
+            lo_l = __ldg(&C.tab.off[row]);
+            ij_l = (u32)max(i, j) | (u32)min(i, j) << 8;
+            if (plen) {
+                len_l = (u32)__ldg(&plen[row]);
+            } else {
+                const u32 all = (u32)(__ldg(&C.tab.off[row + 1]) - lo_l);
+                u32 L = 0, H = all;
+                if (cut <= 0.0) {
+                    L = all;
+                } else if (all && fabs(__ldg(&C.tab.v[lo_l])) >= cut) {
+                    L = 1;
+                    while (L < H) {   // weights descend
+                        const u32 mid = (L + H) >> 1;
+                        if (fabs(__ldg(&C.tab.v[lo_l + mid])) >= cut) L = mid + 1; else H = mid;
+                    }
+                }
+                len_l = L;
+            }
+        }
+        for (unsigned todo = __ballot_sync(0xffffffffu, len_l != 0); todo; todo &= todo - 1) {
+            const int src = __ffs(todo) - 1;
+            const i64 lo = __shfl_sync(0xffffffffu, lo_l, src);
+            const u32 len = __shfl_sync(0xffffffffu, len_l, src);
+            const u32 ij = __shfl_sync(0xffffffffu, ij_l, src);
+            const int ii = ij & 0xff, jj = ij >> 8;
+            u64 ha = R.a, hb = R.b;   // the bra without the pair
+            if (ii & 1) hb &= ~(1ull << (ii >> 1)); else ha &= ~(1ull << (ii >> 1));
+            if (jj & 1) hb &= ~(1ull << (jj >> 1)); else ha &= ~(1ull << (jj >> 1));
+            for (u32 e0 = 0; e0 < len; e0 += 32) {
                 Cand c;
-                const i64 e = e0 + lane;
+                const u32 e = e0 + lane;
                 c.valid = e < len;
                 c.single = false;
                 c.a = R.a;
@@ -253,6 +320,7 @@ __device__ __forceinline__ void enumerate_row(const CtxView& C, const WarpRow& R
                 c.h = 0.0;
                 if (c.valid) {
                     const u16 ab = __ldg(&C.tab.ab[lo + e]);
+                    const double v = __ldg(&C.tab.v[lo + e]);
                     const int A = ab & 0xff, B = ab >> 8;
                     const u64 ma = 1ull << (A >> 1), mb = 1ull << (B >> 1);
                     const bool occA = ((A & 1) ? R.b : R.a) & ma;
@@ -260,20 +328,50 @@ __device__ __forceinline__ void enumerate_row(const CtxView& C, const WarpRow& R
                     if (occA || occB) {
                         c.valid = false;
                     } else {
-                        u64 ka = R.a, kb = R.b;
-                        if (ii & 1) kb &= ~(1ull << (ii >> 1)); else ka &= ~(1ull << (ii >> 1));
-                        if (jj & 1) kb &= ~(1ull << (jj >> 1)); else ka &= ~(1ull << (jj >> 1));
-                        if (A & 1) kb |= ma; else ka |= ma;
-                        if (B & 1) kb |= mb; else ka |= mb;
-                        c.a = ka;
-                        c.b = kb;
-                        c.h = double_elem(R.a, R.b, ii, jj, A, B, __ldg(&C.tab.v[lo + e]));
+                        c.a = ha | ((A & 1) ? 0ull : ma) | ((B & 1) ? 0ull : mb);
+                        c.b = hb | ((A & 1) ? ma : 0ull) | ((B & 1) ? mb : 0ull);
+                        c.h = double_elem(R.a, R.b, ii, jj, A, B, v);
                     }
                 }
                 sink.step(c);
             }
         }
     }
+}
+
+// Part `part` of `parts` of a row, in candidate order over the parts: the
+// singles, then equal shares of the occupied pairs (one part holds all).
+// Spaces of fewer rows than the GPU has warps are cut so (row_parts).
+template <class Sink>
+__device__ __forceinline__ void enumerate_row(const CtxView& C, const WarpRow& R,
+                                              const i64* plen, double cut, Sink& sink,
+                                              int part = 0, int parts = 1) {
+    if (part == 0) enumerate_singles(C, R, sink);
+    const int np = R.ne * (R.ne - 1) / 2;
+    if (parts == 1) enumerate_pairs(C, R, plen, cut, sink, 0, np);
+    else if (part > 0)
+        enumerate_pairs(C, R, plen, cut, sink, (int)((i64)np * (part - 1) / (parts - 1)),
+                        (int)((i64)np * part / (parts - 1)));
+}
+
+// Parts per row: enough for four units of work per warp, at most one of eight
+// pairs each (a unit sets its row up again, ~1 us).  At 403 rows of 24 orbitals
+// a warp per row left nine in ten warps idle: a count and a fill pass 5.06 ms so,
+// 0.48 cut (2,241 rows of 13 orbitals 0.65 -> 0.31, PT2 at 3,001 rows of 20
+// orbitals 3.50 -> 1.49).
+inline int row_parts(i64 n, i64 warps, int n_orb) {
+    if (n <= 0 || n >= 2 * warps) return 1;
+    const i64 want = (4 * warps + n - 1) / n;
+    const i64 pairs = (i64)n_orb * (n_orb - 1) / 2;   // of a half-filled row
+    const i64 parts = std::min<i64>(want, pairs / 8 + 1) + 1;
+    return parts <= 2 ? 1 : (int)std::min<i64>(parts, 128);
+}
+
+// rowptr[r] = first offset of row r's parts, r <= n.
+__global__ static void k_first_parts(const i64* off, int parts, i64 n, i64* rowptr) {
+    for (i64 r = blockIdx.x * (i64)blockDim.x + threadIdx.x; r <= n;
+         r += (i64)gridDim.x * blockDim.x)
+        rowptr[r] = off[r * parts];
 }
 
 // All candidates of the bra in the order get_local_conn visits them without

@@ -41,6 +41,16 @@ i64 rd(const i64* d, cudaStream_t s) {
     return v;
 }
 
+// The warp's next unit of work, its row and part; -1 when none is left.
+__device__ __forceinline__ int next_unit(int* ctr, i64 n, int parts, int& r, int& part) {
+    int u = 0;
+    if ((threadIdx.x & 31) == 0) u = atomicAdd(ctr, 1);
+    u = __shfl_sync(0xffffffffu, u, 0);
+    r = u / parts;
+    part = u % parts;
+    return u < n * parts ? u : -1;
+}
+
 __device__ __forceinline__ i64 choose2(int m) { return m < 2 ? 0 : (i64)m * (m - 1) / 2; }
 
 // k-th pair (x < y) of m items in the order x ascending, y ascending.
@@ -138,6 +148,7 @@ __global__ void __launch_bounds__(kW * 32) k_comb(CombParams P) {
 // (dynamic: also |h psi_i| >= eps1), heat-bath doubles with w >= cut and
 // no element test; kets in V are dropped.
 struct ScrParams {
+    int parts;           // units of work per row (enumerate_row); cnt and off are per unit
     CtxView C;
     const u64* V;
     i64 n;
@@ -185,10 +196,9 @@ __global__ void __launch_bounds__(kW * 32) k_screened(ScrParams P) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WarpRow& R = rows[w];
     for (;;) {
-        int r = 0;
-        if (lane == 0) r = atomicAdd(P.next_row, 1);
-        r = __shfl_sync(0xffffffffu, r, 0);
-        if (r >= P.n) break;
+        int r, part;
+        const int unit = next_unit(P.next_row, P.n, P.parts, r, part);
+        if (unit < 0) break;
         load_row(R, P.V[2 * (i64)r], P.V[2 * (i64)r + 1], P.n_orb);
         double ps = 0.0, cut = P.cut;
         if (P.dynamic) {
@@ -196,11 +206,11 @@ __global__ void __launch_bounds__(kW * 32) k_screened(ScrParams P) {
             cut = fmax(P.eps1 / fmax(fabs(ps), kAmpDelta), P.cut);
         }
         ScrSink<FILL> sink(P, ps);
-        if (FILL) sink.wpos = P.off[r];
-        enumerate_row(P.C, R, nullptr, cut, sink);
+        if (FILL) sink.wpos = P.off[unit];
+        enumerate_row(P.C, R, nullptr, cut, sink, part, P.parts);
         if (!FILL) {
             const u32 c = __reduce_add_sync(0xffffffffu, sink.c);
-            if (lane == 0) P.cnt[r] = c;
+            if (lane == 0) P.cnt[unit] = c;
         }
         __syncwarp();
     }
@@ -257,6 +267,7 @@ int grid_of(const void* kern, int device, int block) {
 // local connections
 // ---------------------------------------------------------------------------
 struct ConnParams {
+    int parts;           // units of work per row (enumerate_row); cnt and off are per unit
     CtxView C;
     const u64* V;
     i64 n;
@@ -301,17 +312,16 @@ __global__ void __launch_bounds__(kW * 32) k_conn(ConnParams P) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WarpRow& R = rows[w];
     for (;;) {
-        int r = 0;
-        if (lane == 0) r = atomicAdd(P.next_row, 1);
-        r = __shfl_sync(0xffffffffu, r, 0);
-        if (r >= P.n) break;
+        int r, part;
+        const int unit = next_unit(P.next_row, P.n, P.parts, r, part);
+        if (unit < 0) break;
         const u64 a = P.V[2 * (i64)r], b = P.V[2 * (i64)r + 1];
         load_row(R, a, b, P.n_orb);
         ConnSink<FILL> sink(P);
         const double d = P.diag[r];
-        const bool dk = fabs(d) > kElemThresh;     // local_conn.cpp:61-66
+        const bool dk = part == 0 && fabs(d) > kElemThresh;     // local_conn.cpp:61-66
         if (FILL) {
-            sink.wpos = P.off[r];
+            sink.wpos = P.off[unit];
             if (dk) {
                 if (lane == 0) {
                     P.keys[sink.wpos] = make_ulonglong2(a, b);
@@ -323,10 +333,10 @@ __global__ void __launch_bounds__(kW * 32) k_conn(ConnParams P) {
             sink.c = 1;
         }
         if (P.full_order) enumerate_row_full(P.C, R, sink);
-        else enumerate_row(P.C, R, P.plen, P.cut, sink);
+        else enumerate_row(P.C, R, P.plen, P.cut, sink, part, P.parts);
         if (!FILL) {
             const u32 c = __reduce_add_sync(0xffffffffu, sink.c);
-            if (lane == 0) P.cnt[r] = c;
+            if (lane == 0) P.cnt[unit] = c;
         }
         __syncwarp();
     }
@@ -350,6 +360,7 @@ __global__ void k_plen(PairTableView T, i64 nrows, double cut, i64* plen) {
 // EN-PT2 external part: (key, h c_i) contributions of kets outside V
 // ---------------------------------------------------------------------------
 struct Pt2Params {
+    int parts;           // units of work per row (enumerate_row); cnt and off are per unit
     CtxView C;
     const u64* V;
     i64 n;
@@ -396,27 +407,26 @@ __global__ void __launch_bounds__(kW * 32) k_pt2ext(Pt2Params P) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WarpRow& R = rows[w];
     for (;;) {
-        int r = 0;
-        if (lane == 0) r = atomicAdd(P.next_row, 1);
-        r = __shfl_sync(0xffffffffu, r, 0);
-        if (r >= P.n) break;
+        int r, part;
+        const int unit = next_unit(P.next_row, P.n, P.parts, r, part);
+        if (unit < 0) break;
         const double ci = P.coeff[r];
         if (ci * ci < 1e-15) {                    // local_conn.cpp:300
-            if (!FILL && lane == 0) P.cnt[r] = 0;
+            if (!FILL && lane == 0) P.cnt[unit] = 0;
             continue;
         }
         load_row(R, P.V[2 * (i64)r], P.V[2 * (i64)r + 1], P.n_orb);
         Pt2Sink<FILL> sink(P, ci);
-        if (FILL) sink.wpos = P.off[r];
+        if (FILL) sink.wpos = P.off[unit];
         if (P.use_hb) {
             const double tau = P.eps1 / fmax(fabs(ci), kAmpDelta);   // :368-372
-            enumerate_row(P.C, R, nullptr, fmax(tau, P.cut_floor), sink);
+            enumerate_row(P.C, R, nullptr, fmax(tau, P.cut_floor), sink, part, P.parts);
         } else {
-            enumerate_row(P.C, R, P.plen_full, 0.0, sink);
+            enumerate_row(P.C, R, P.plen_full, 0.0, sink, part, P.parts);
         }
         if (!FILL) {
             const u32 c = __reduce_add_sync(0xffffffffu, sink.c);
-            if (lane == 0) P.cnt[r] = c;
+            if (lane == 0) P.cnt[unit] = c;
         }
         __syncwarp();
     }
@@ -530,11 +540,16 @@ void gen_dets(dnq_ctx_s* ctx, const u64* Vd, i64 n, int n_orb, const double* psi
     DetMap mapV;
     if (mode >= 0) build_detmap(mapV, Vd, n, true, s);
     DBuf<int> next(1, s);
-    DBuf<u32> cnt(n + 1, s);
-    DBuf<i64> off(n + 1, s);
-    DNQ_CUDA(cudaMemsetAsync(cnt.p + n, 0, 4, s));
+    DBuf<u32> cnt;
+    DBuf<i64> off;
     DBuf<ulonglong2> keys;
+    auto units = [&](i64 nu) {   // counts and offsets of nu units of work
+        cnt.alloc(nu + 1, s);
+        off.alloc(nu + 1, s);
+        DNQ_CUDA(cudaMemsetAsync(cnt.p + nu, 0, 4, s));
+    };
     if (mode <= 0) {
+        units(n);
         CombParams P{};
         P.V = Vd;
         P.n = n;
@@ -569,13 +584,16 @@ void gen_dets(dnq_ctx_s* ctx, const u64* Vd, i64 n, int n_orb, const double* psi
         P.eps1 = eps1;
         P.cut = mode == 2 ? ctx->hb_thr : hb_cutoff(ctx, eps1);
         P.next_row = next.p;
-        P.cnt = cnt.p;
         const int grid = grid_of((const void*)k_screened<false>, device, kW * 32);
+        P.parts = row_parts(n, (i64)grid * kW, n_orb);
+        const i64 nu = n * P.parts;
+        units(nu);
+        P.cnt = cnt.p;
         DNQ_CUDA(cudaMemsetAsync(next.p, 0, 4, s));
         k_screened<false><<<grid, kW * 32, 0, s>>>(P);
         DNQ_CHECK_LAUNCH();
-        scan_ex(cnt.p, off.p, n + 1, s);
-        const i64 tot = rd(off.p + n, s);
+        scan_ex(cnt.p, off.p, nu + 1, s);
+        const i64 tot = rd(off.p + nu, s);
         keys.alloc(tot, s);
         P.off = off.p;
         P.keys = keys.p;
@@ -605,10 +623,15 @@ void local_connections(dnq_ctx_s* ctx, const u64* Vd, i64 n, int n_orb, bool use
     DBuf<i64> plen(ctx->tab.n_rows, s);
     k_plen<<<gsz(ctx->tab.n_rows), 256, 0, s>>>(ctx->view().tab, ctx->tab.n_rows, cut, plen.p);
     DNQ_CHECK_LAUNCH();
+    const int grid = grid_of((const void*)k_conn<false>, ctx->device, kW * 32);
+    const int parts = use_hb ? row_parts(n, (i64)grid * kW, n_orb) : 1;
+    const i64 nu = n * parts;
     DBuf<int> next(1, s);
-    DBuf<u32> cnt(n + 1, s);
-    DNQ_CUDA(cudaMemsetAsync(cnt.p + n, 0, 4, s));
+    DBuf<u32> cnt(nu + 1, s);
+    DBuf<i64> off(nu + 1, s);
+    DNQ_CUDA(cudaMemsetAsync(cnt.p + nu, 0, 4, s));
     ConnParams P{};
+    P.parts = parts;
     P.C = ctx->view();
     P.V = Vd;
     P.n = n;
@@ -620,19 +643,20 @@ void local_connections(dnq_ctx_s* ctx, const u64* Vd, i64 n, int n_orb, bool use
     P.full_order = !use_hb;
     P.next_row = next.p;
     P.cnt = cnt.p;
-    const int grid = grid_of((const void*)k_conn<false>, ctx->device, kW * 32);
     DNQ_CUDA(cudaMemsetAsync(next.p, 0, 4, s));
     k_conn<false><<<grid, kW * 32, 0, s>>>(P);
     DNQ_CHECK_LAUNCH();
-    scan_ex(cnt.p, H->vv.rowptr.p, n + 1, s);
-    const i64 tot = rd(H->vv.rowptr.p + n, s);
+    scan_ex(cnt.p, off.p, nu + 1, s);
+    k_first_parts<<<gsz(n + 1), 256, 0, s>>>(off.p, parts, n, H->vv.rowptr.p);
+    DNQ_CHECK_LAUNCH();
+    const i64 tot = rd(off.p + nu, s);
     require(tot <= (i64)0x7fffffff, DNQ_ERR_OVERFLOW,
             "local connections exceed the int32 offsets of the reference format");
     H->vv.nnz = tot;
     H->n_p = tot;
     H->vv.val.alloc(tot, s);
     DBuf<ulonglong2> keys(tot, s);
-    P.off = H->vv.rowptr.p;
+    P.off = off.p;
     P.keys = keys.p;
     P.vals = H->vv.val.p;
     DNQ_CUDA(cudaMemsetAsync(next.p, 0, 4, s));
@@ -662,11 +686,15 @@ void pt2(dnq_ctx_s* ctx, const u64* Vd, i64 n, const double* cd, int n_orb, doub
     k_plen<<<gsz(ctx->tab.n_rows), 256, 0, s>>>(ctx->view().tab, ctx->tab.n_rows,
                                                  full_cutoff(), plen.p);
     DNQ_CHECK_LAUNCH();
+    const int grid = grid_of((const void*)k_pt2ext<false>, ctx->device, kW * 32);
+    const int parts = row_parts(n, (i64)grid * kW, n_orb);
+    const i64 units = n * parts;
     DBuf<int> next(1, s);
-    DBuf<u32> cnt(n + 1, s);
-    DBuf<i64> off(n + 1, s);
-    DNQ_CUDA(cudaMemsetAsync(cnt.p + n, 0, 4, s));
+    DBuf<u32> cnt(units + 1, s);
+    DBuf<i64> off(units + 1, s);
+    DNQ_CUDA(cudaMemsetAsync(cnt.p + units, 0, 4, s));
     Pt2Params P{};
+    P.parts = parts;
     P.C = ctx->view();
     P.V = Vd;
     P.n = n;
@@ -679,12 +707,11 @@ void pt2(dnq_ctx_s* ctx, const u64* Vd, i64 n, const double* cd, int n_orb, doub
     P.plen_full = plen.p;
     P.next_row = next.p;
     P.cnt = cnt.p;
-    const int grid = grid_of((const void*)k_pt2ext<false>, ctx->device, kW * 32);
     DNQ_CUDA(cudaMemsetAsync(next.p, 0, 4, s));
     k_pt2ext<false><<<grid, kW * 32, 0, s>>>(P);
     DNQ_CHECK_LAUNCH();
-    scan_ex(cnt.p, off.p, n + 1, s);
-    const i64 tot = rd(off.p + n, s);
+    scan_ex(cnt.p, off.p, units + 1, s);
+    const i64 tot = rd(off.p + units, s);
     DBuf<ulonglong2> keys(tot, s), ks(tot, s);
     DBuf<double> vals(tot, s), vs(tot, s);
     P.off = off.p;

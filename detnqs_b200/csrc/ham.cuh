@@ -21,14 +21,15 @@ struct Csr {
     DBuf<i64> rowend;    // arena form only
     DBuf<u32> col;
     DBuf<double> val;
-    DBuf<float> val32;   // optional FP32 off-diagonal copy (ready when as long as val)
+    DBuf<float> val32;   // optional FP32 off-diagonal copy (ready when span() long)
     i64 nr = 0, nc = 0, nnz = 0;
     bool sorted = true;   // columns ascending inside each row
     bool arena = false;
+    i64 used = -1;        // arena form: slots handed out (the arrays may be longer)
     const i64* row_start() const { return rowptr.p; }
     const i64* row_end() const { return arena ? rowend.p : rowptr.p + 1; }
-    i64 span() const { return (i64)col.n; }
-    bool f32_ready() const { return val32.n == val.n; }
+    i64 span() const { return arena && used >= 0 ? used : (i64)col.n; }
+    bool f32_ready() const { return (i64)val32.n == span(); }
     size_t bytes() const {
         return rowptr.bytes() + rowend.bytes() + col.bytes() + val.bytes() + val32.bytes();
     }

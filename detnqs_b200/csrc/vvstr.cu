@@ -2196,7 +2196,11 @@ i64 run_vv(const Loc& L, i64 nrows, i64 cap_hint, int device, cudaStream_t s, Cs
         }
         M.col = std::move(acol);
         M.val = std::move(aval);
-        if (f32_in_build) M.val32 = std::move(av32);
+        M.used = used;
+        if (f32_in_build) {
+            M.val32 = std::move(av32);
+            M.used = (i64)M.val32.n;   // the copy is as long as the arrays
+        }
         M.arena = true;
     } else if (!hov) {
         M.rowptr.alloc(nrows + 1, s);
@@ -2339,6 +2343,7 @@ void ensure_compact(Csr& m, cudaStream_t s) {
     if (f32) m.val32 = std::move(v32);
     else m.val32.release();
     m.arena = false;
+    m.used = -1;
 }
 
 void launch_check_orbitals(const u64* d, i64 n, int n_orb, unsigned long long* bad,

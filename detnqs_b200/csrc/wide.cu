@@ -21,7 +21,7 @@
 #include <memory>
 #include <vector>
 
-#include "context.cuh"
+#include "gen.cuh"
 #include "ham.cuh"
 #include "prim.cuh"
 
@@ -66,28 +66,35 @@ struct WRow {
     u8 occa[128], occb[128], vira[128], virb[128];
 };
 
+// One lane per orbital (load_row).
 __device__ __forceinline__ void load_wrow(WRow& R, M2 a, M2 b, int n_orb) {
     const int lane = threadIdx.x & 31;
+    const int na = __popcll(a.lo) + __popcll(a.hi), nb = __popcll(b.lo) + __popcll(b.hi);
+    for (int o = lane; o < n_orb; o += 32) {
+        const M2 m = mask_below(o);
+        const int oa = __popcll(a.lo & m.lo) + __popcll(a.hi & m.hi);
+        const int ob = __popcll(b.lo & m.lo) + __popcll(b.hi & m.hi);
+        if (bit(a, o)) {
+            R.occa[oa] = (u8)o;
+            R.occ[oa] = (u8)(2 * o);
+        } else {
+            R.vira[o - oa] = (u8)o;
+        }
+        if (bit(b, o)) {
+            R.occb[ob] = (u8)o;
+            R.occ[na + ob] = (u8)(2 * o + 1);
+        } else {
+            R.virb[o - ob] = (u8)o;
+        }
+    }
     if (lane == 0) {
         R.a = a;
         R.b = b;
-        int k = 0, t = 0;
-        for (int o = 0; o < n_orb; ++o)
-            if (bit(a, o)) { R.occa[t++] = (u8)o; R.occ[k++] = (u8)(2 * o); }
-        R.na = t;
-        t = 0;
-        for (int o = 0; o < n_orb; ++o)
-            if (bit(b, o)) { R.occb[t++] = (u8)o; R.occ[k++] = (u8)(2 * o + 1); }
-        R.nb = t;
-        R.ne = k;
-        t = 0;
-        for (int o = 0; o < n_orb; ++o)
-            if (!bit(a, o)) R.vira[t++] = (u8)o;
-        R.nva = t;
-        t = 0;
-        for (int o = 0; o < n_orb; ++o)
-            if (!bit(b, o)) R.virb[t++] = (u8)o;
-        R.nvb = t;
+        R.na = na;
+        R.nb = nb;
+        R.ne = na + nb;
+        R.nva = n_orb - na;
+        R.nvb = n_orb - nb;
     }
     __syncwarp();
 }
@@ -120,45 +127,10 @@ __device__ double diag2(const CtxView& C, const M2& a, const M2& b) {
     return one + two;
 }
 
-// Single h -> p in spin s (ham_eval.cpp:88-115): h1 first, then the other
-// occupied orbitals, alpha ascending then beta ascending.
-// e + arr[occ[t]] for t = 0..cnt-1 except occ[t] == skip, added in t order;
-// the loads are issued eight at a time ahead of their additions.
-__device__ __forceinline__ double add_occ(double e, const double* arr, const u8* occ, int cnt,
-                                          int skip) {
-    int t = 0;
-    for (; t + 8 <= cnt; t += 8) {
-        double v[8];
-        int o[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            o[q] = occ[t + q];
-            v[q] = __ldg(&arr[o[q]]);
-        }
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-            if (o[q] != skip) e += v[q];
-    }
-    for (; t < cnt; ++t)
-        if (occ[t] != skip) e += arr[occ[t]];
-    return e;
-}
-
+// Single h -> p in spin s of the row in R.
 __device__ __forceinline__ double single2(const CtxView& C, const WRow& R, int s, int h, int p) {
-    const int n = C.n;
-    double e = C.h1[h * n + p];
-    const size_t base = ((size_t)h * n + p) * n;
-    const double* ss = C.sss + base;
-    const double* os = C.sos + base;
-    if (s == 0) {
-        e = add_occ(e, ss, R.occa, R.na, h);
-        e = add_occ(e, os, R.occb, R.nb, -1);
-    } else {
-        e = add_occ(e, os, R.occa, R.na, -1);
-        e = add_occ(e, ss, R.occb, R.nb, h);
-    }
-    const int perm = between2(s ? R.b : R.a, h, p);
-    return (perm & 1) ? -e : e;
+    const double e = single_sum(C, R.occa, R.na, R.occb, R.nb, s, h, p);
+    return (between2(s ? R.b : R.a, h, p) & 1) ? -e : e;
 }
 
 // Double i,j -> a,b (spin-orbitals, i > j, a > b) from v = <ij||ab>, with
@@ -183,26 +155,6 @@ __device__ __forceinline__ double double2(const M2& ba, const M2& bb, int i, int
         perm = between2(ba, ha, pa) + between2(bb, hb, pb);
     }
     return (perm & 1) ? -raw : raw;
-}
-
-__device__ __forceinline__ i64 prefix_len(const double* v, i64 len, double cut) {
-    if (cut <= 0.0 || len == 0) return len;
-    const int lane = threadIdx.x & 31;
-    i64 lo = 0, hi = len;
-    while (hi - lo > 32) {
-        const i64 step = (hi - lo + 31) / 32;
-        const i64 x = lo + lane * step;
-        const bool ok = x < hi && fabs(v[x]) >= cut;
-        const int k = __popc(__ballot_sync(0xffffffffu, ok));
-        if (k == 0) return lo;
-        const i64 nlo = lo + (i64)(k - 1) * step + 1;
-        const i64 nhi = min(hi, lo + (i64)k * step);
-        lo = nlo;
-        hi = nhi;
-    }
-    const i64 x = lo + lane;
-    const bool ok = x < hi && fabs(v[x]) >= cut;
-    return lo + __popc(__ballot_sync(0xffffffffu, ok));
 }
 
 __device__ __forceinline__ u64 mix(u64 x) {
@@ -461,50 +413,62 @@ __global__ void __launch_bounds__(kWW * 32) k_wide_build(WParams P) {
                 emit(valid, ka, kb, h);
             }
         }
-        // heat-bath doubles over occupied pairs (ham_utils.hpp:280-313)
+        // heat-bath doubles over occupied pairs (ham_utils.hpp:280-313), the
+        // prefixes of 32 pairs searched side by side (enumerate_pairs)
         const int p_lo = seg_lo == 0 ? 0 : (int)seg_lo - 1;
         const int p_hi = (int)seg_hi - 1;
-        int x = 1, y = 0;
-        {
-            int xx = (int)((1.0 + sqrt(1.0 + 8.0 * p_lo)) * 0.5);
-            while (xx * (xx - 1) / 2 > p_lo) --xx;
-            while ((xx + 1) * xx / 2 <= p_lo) ++xx;
-            x = max(xx, 1);
-            y = p_lo - x * (x - 1) / 2;
-        }
-        for (int p = p_lo; p < p_hi; ++p) {
-            const int i = R.occ[x];
-            const int jj0 = R.occ[y];
-            const i64 row = pair_row(i, jj0);
-            const i64 lo = __ldg(&P.C.tab.off[row]);
-            const i64 len = prefix_len(P.C.tab.v + lo, __ldg(&P.C.tab.off[row + 1]) - lo, cut);
-            const int ii = max(i, jj0), jj = min(i, jj0);
-            for (i64 e0 = 0; e0 < len; e0 += 32) {
-                const i64 e = e0 + lane;
-                bool valid = e < len;
-                M2 ka = R.a, kb = R.b;
-                double h = 0.0;
-                if (valid) {
-                    const u16 ab = __ldg(&P.C.tab.ab[lo + e]);
-                    const int A = ab & 0xff, B = ab >> 8;
-                    const bool oA = (A >> 1) >= P.n_orb || bit((A & 1) ? R.b : R.a, A >> 1);
-                    const bool oB = (B >> 1) >= P.n_orb || bit((B & 1) ? R.b : R.a, B >> 1);
-                    if (oA || oB) {
-                        valid = false;
-                    } else {
-                        M2* w[2] = {&ka, &kb};
-                        flip(*w[ii & 1], ii >> 1);
-                        flip(*w[jj & 1], jj >> 1);
-                        flip(*w[A & 1], A >> 1);
-                        flip(*w[B & 1], B >> 1);
-                        h = double2(R.a, R.b, ii, jj, A, B, __ldg(&P.C.tab.v[lo + e]));
+        for (int p0 = p_lo; p0 < p_hi; p0 += 32) {
+            i64 lo_l = 0;
+            u32 len_l = 0, ij_l = 0;
+            if (p0 + lane < p_hi) {
+                int x, y;
+                pair_of(p0 + lane, x, y);
+                const int i = R.occ[x], j = R.occ[y];
+                const i64 row = pair_row(i, j);
+                lo_l = __ldg(&P.C.tab.off[row]);
+                ij_l = (u32)max(i, j) | (u32)min(i, j) << 8;
+                const u32 all = (u32)(__ldg(&P.C.tab.off[row + 1]) - lo_l);
+                if (cut <= 0.0) {
+                    len_l = all;
+                } else if (all && fabs(__ldg(&P.C.tab.v[lo_l])) >= cut) {
+                    u32 L = 1, H = all;
+                    while (L < H) {   // weights descend
+                        const u32 mid = (L + H) >> 1;
+                        if (fabs(__ldg(&P.C.tab.v[lo_l + mid])) >= cut) L = mid + 1; else H = mid;
                     }
+                    len_l = L;
                 }
-                emit(valid, ka, kb, h);
             }
-            if (++y == x) {
-                ++x;
-                y = 0;
+            for (unsigned todo = __ballot_sync(0xffffffffu, len_l != 0); todo; todo &= todo - 1) {
+                const int src = __ffs(todo) - 1;
+                const i64 lo = __shfl_sync(0xffffffffu, lo_l, src);
+                const u32 len = __shfl_sync(0xffffffffu, len_l, src);
+                const u32 ij = __shfl_sync(0xffffffffu, ij_l, src);
+                const int ii = ij & 0xff, jj = ij >> 8;
+                for (u32 e0 = 0; e0 < len; e0 += 32) {
+                    const u32 e = e0 + lane;
+                    bool valid = e < len;
+                    M2 ka = R.a, kb = R.b;
+                    double h = 0.0;
+                    if (valid) {
+                        const u16 ab = __ldg(&P.C.tab.ab[lo + e]);
+                        const double v = __ldg(&P.C.tab.v[lo + e]);
+                        const int A = ab & 0xff, B = ab >> 8;
+                        const bool oA = (A >> 1) >= P.n_orb || bit((A & 1) ? R.b : R.a, A >> 1);
+                        const bool oB = (B >> 1) >= P.n_orb || bit((B & 1) ? R.b : R.a, B >> 1);
+                        if (oA || oB) {
+                            valid = false;
+                        } else {
+                            M2* w[2] = {&ka, &kb};
+                            flip(*w[ii & 1], ii >> 1);
+                            flip(*w[jj & 1], jj >> 1);
+                            flip(*w[A & 1], A >> 1);
+                            flip(*w[B & 1], B >> 1);
+                            h = double2(R.a, R.b, ii, jj, A, B, v);
+                        }
+                    }
+                    emit(valid, ka, kb, h);
+                }
             }
         }
         if (!FILL) {
