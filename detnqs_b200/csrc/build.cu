@@ -19,6 +19,7 @@
 
 #include "gen.cuh"
 #include "ham.cuh"
+#include "hostcopy.cuh"
 #include "prim.cuh"
 
 namespace dnq {
@@ -882,16 +883,6 @@ int dnq_ham_info(dnq_ham_t h, int64_t* info) {
 
 }  // extern "C"
 
-namespace dnq {
-namespace {
-__global__ void k_expand_rows(const i64* rowptr, i64 nr, u32* rows) {
-    for (i64 r = blockIdx.x * (i64)blockDim.x + threadIdx.x; r < nr;
-         r += (i64)gridDim.x * blockDim.x)
-        for (i64 k = rowptr[r]; k < rowptr[r + 1]; ++k) rows[k] = (u32)r;
-}
-}  // namespace
-}  // namespace dnq
-
 extern "C" {
 
 int dnq_ham_copy_coo(dnq_ham_t h, int block, uint32_t* rows, uint32_t* cols, double* vals,
@@ -903,15 +894,16 @@ int dnq_ham_copy_coo(dnq_ham_t h, int block, uint32_t* rows, uint32_t* cols, dou
     Csr& m = block == 0 ? h->vv : h->vp;
     if (m.nnz == 0) return DNQ_OK;
     ensure_sorted(m, s);
+    HostCopies out(s);
+    DBuf<u32> r;
     if (rows) {
-        DBuf<u32> r(m.nnz, s);
-        k_expand_rows<<<grid_for(m.nr), 256, 0, s>>>(m.rowptr.p, m.nr, r.p);
-        DNQ_CHECK_LAUNCH();
-        copy_out(rows, r.p, m.nnz, s);
-        DNQ_CUDA(cudaStreamSynchronize(s));
+        r.alloc(m.nnz, s);
+        prim::rows_of(m.rowptr.p, m.nr, m.nnz, r.p, s);
+        out.add(rows, r.p, m.nnz);
     }
-    copy_out(cols, m.col.p, m.nnz, s);
-    copy_out(vals, m.val.p, m.nnz, s);
+    out.add(cols, m.col.p, m.nnz);
+    out.add(vals, m.val.p, m.nnz);
+    out.run();
     DNQ_CUDA(cudaStreamSynchronize(s));
     DNQ_API_END
 }
@@ -929,8 +921,10 @@ int dnq_ham_copy_csr(dnq_ham_t h, int block, int64_t* row_ptr, uint32_t* cols, d
         const int64_t z = 0;
         DNQ_CUDA(cudaMemcpyAsync(row_ptr, &z, 8, cudaMemcpyDefault, s));
     }
-    copy_out(cols, m.col.p, m.nnz, s);
-    copy_out(vals, m.val.p, m.nnz, s);
+    HostCopies out(s);
+    out.add(cols, m.col.p, m.nnz);
+    out.add(vals, m.val.p, m.nnz);
+    out.run();
     DNQ_CUDA(cudaStreamSynchronize(s));
     DNQ_API_END
 }
@@ -940,7 +934,9 @@ int dnq_ham_copy_dets_p(dnq_ham_t h, uint64_t* dets, void* stream) {
     require(h != nullptr, DNQ_ERR_INVALID, "null argument");
     DeviceGuard g(h->device);
     cudaStream_t s = (cudaStream_t)stream;
-    copy_out(dets, (const uint64_t*)h->dets_p.p, 2 * (i64)h->words * h->n_p, s);
+    HostCopies out(s);
+    out.add(dets, (const uint64_t*)h->dets_p.p, 2 * (i64)h->words * h->n_p);
+    out.run();
     DNQ_CUDA(cudaStreamSynchronize(s));
     DNQ_API_END
 }

@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "hostcopy.cuh"
 
 namespace dnq {
 
@@ -88,6 +89,7 @@ struct PairTable {
 }  // namespace dnq
 
 struct dnq_ctx_s {
+    dnq::HostSlots slots;   // keeps the staged copies' page-locked memory
     int device = 0;
     int n = 0;
     int nso = 0;

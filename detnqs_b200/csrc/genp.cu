@@ -11,6 +11,7 @@
 
 #include "gen.cuh"
 #include "ham.cuh"
+#include "hostcopy.cuh"
 #include "prim.cuh"
 
 namespace dnq {
@@ -810,8 +811,10 @@ int dnq_conn_copy(dnq_ham_t h, int32_t* offsets, uint64_t* dets, double* values,
         DNQ_CUDA(cudaMemcpyAsync(offsets, o.data(), (h->n_v + 1) * 4, cudaMemcpyDefault, s));
         DNQ_CUDA(cudaStreamSynchronize(s));
     }
-    copy_out(dets, (const uint64_t*)h->dets_p.p, 2 * h->n_p, s);
-    copy_out(values, h->vv.val.p, h->vv.nnz, s);
+    HostCopies out(s);
+    out.add(dets, (uint64_t*)h->dets_p.p, 2 * h->n_p);
+    out.add(values, h->vv.val.p, h->vv.nnz);
+    out.run();
     DNQ_CUDA(cudaStreamSynchronize(s));
     DNQ_API_END
 }

@@ -711,6 +711,49 @@ void segment_sums(const T* v, const i64* rp, i64 nseg, Tout* out, cudaStream_t s
 }
 
 // ---------------------------------------------------------------------------
+// Row of every entry of a CSR block
+// ---------------------------------------------------------------------------
+
+// Four consecutive entries per thread: one binary search of the row pointers
+// for the first, the others walk on from its row, and one 16-byte store.  (A
+// thread per row wrote the rows of a 13-million-entry block in 2.3 ms, a
+// search per entry of 4.35e6 took 47 us.)
+__global__ void k_rows_of(const i64* rowptr, i64 nr, i64 nnz, u32* rows) {
+    for (i64 k = 4 * (blockIdx.x * (i64)blockDim.x + threadIdx.x); k < nnz;
+         k += 4 * (i64)gridDim.x * blockDim.x) {
+        i64 lo = 0, hi = nr;   // last r with rowptr[r] <= k
+        while (hi - lo > 1) {
+            const i64 mid = (lo + hi) >> 1;
+            if (__ldg(&rowptr[mid]) <= k) lo = mid; else hi = mid;
+        }
+        u32 r[4];
+        i64 end = __ldg(&rowptr[lo + 1]);
+        const int m = (int)min((i64)4, nnz - k);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (q < m)
+                while (k + q >= end) end = __ldg(&rowptr[++lo + 1]);   // empty rows too
+            r[q] = (u32)lo;
+        }
+        if (m == 4) {   // rows starts an allocation and k is a multiple of 4
+            *reinterpret_cast<uint4*>(rows + k) = make_uint4(r[0], r[1], r[2], r[3]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (q < m) rows[k + q] = r[q];
+        }
+    }
+}
+
+// rows[k] = the row of entry k < nnz; rows 16-byte aligned.
+inline void rows_of(const i64* rowptr, i64 nr, i64 nnz, u32* rows, cudaStream_t s) {
+    if (nnz <= 0) return;
+    const unsigned g = (unsigned)std::min<i64>((nnz + 1023) / 1024, 1 << 20);
+    k_rows_of<<<g, 256, 0, s>>>(rowptr, nr, nnz, rows);
+    DNQ_CHECK_LAUNCH();
+}
+
+// ---------------------------------------------------------------------------
 // Column sort of every row of a CSR block (columns of a row are distinct)
 // ---------------------------------------------------------------------------
 

@@ -17,20 +17,6 @@ void to_f32(const double* x, i64 n, float* o, cudaStream_t s);
 
 namespace {
 
-// Row of every entry: one thread per entry, binary search of the row
-// pointers (rows of any length, no serial walk).
-__global__ void k_rows_of(const i64* rowptr, i64 nr, i64 nnz, u32* rows) {
-    for (i64 k = blockIdx.x * (i64)blockDim.x + threadIdx.x; k < nnz;
-         k += (i64)gridDim.x * blockDim.x) {
-        i64 lo = 0, hi = nr;   // last r with rowptr[r] <= k
-        while (hi - lo > 1) {
-            const i64 mid = (lo + hi) >> 1;
-            if (rowptr[mid] <= k) lo = mid; else hi = mid;
-        }
-        rows[k] = (u32)lo;
-    }
-}
-
 __global__ void k_gather_t(const u32* perm, const u32* rows, const double* val, i64 n,
                            u32* tcol, double* tval) {
     for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
@@ -79,8 +65,7 @@ void transpose_csr(const Csr& a, Csr& t, cudaStream_t s) {
         return;
     }
     DBuf<u32> rows(a.nnz, s), perm2(a.nnz, s), skey(a.nnz, s);
-    k_rows_of<<<gsz(a.nnz), 256, 0, s>>>(a.rowptr.p, a.nr, a.nnz, rows.p);
-    DNQ_CHECK_LAUNCH();
+    prim::rows_of(a.rowptr.p, a.nr, a.nnz, rows.p, s);
     {   // stable by column: rows stay ascending inside each column
         int b = 1;
         while (b < 32 && ((i64)1 << b) < a.nc) ++b;
