@@ -16,6 +16,7 @@
 #include <cmath>
 #include <memory>
 #include <mutex>
+#include <type_traits>
 
 #include "gen.cuh"
 #include "ham.cuh"
@@ -195,37 +196,57 @@ k_build(BuildParams P) {
     }
 }
 
-__global__ void k_unique_flags(const ulonglong2* k, i64 n, u32* flag) {
+__device__ __forceinline__ bool differ(u64 a, u64 b) { return a != b; }
+__device__ __forceinline__ bool differ(const ulonglong2& a, const ulonglong2& b) {
+    return a.x != b.x || a.y != b.y;
+}
+// (alpha, beta) of a key: alpha << n_orb | beta for n_orb <= 32.
+__device__ __forceinline__ ulonglong2 det_of(u64 k, int n_orb) {
+    return make_ulonglong2(k >> n_orb, k & low_mask(n_orb));
+}
+__device__ __forceinline__ ulonglong2 det_of(const ulonglong2& k, int) { return k; }
+
+template <class K>
+__global__ void k_unique_flags(const K* k, i64 n, u32* flag) {
     for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
          t += (i64)gridDim.x * blockDim.x)
-        flag[t] = (t == 0 || k[t].x != k[t - 1].x || k[t].y != k[t - 1].y) ? 1u : 0u;
+        flag[t] = t == 0 || differ(k[t], k[t - 1]) ? 1u : 0u;
 }
 
-__global__ void k_unique_scatter(const ulonglong2* k, const u32* perm, const u32* runid,
-                                 i64 n, unsigned long long* pdets, u32* col) {
+template <class K>
+__global__ void k_unique_dets(const K* k, const u32* runid, i64 n, int n_orb,
+                              unsigned long long* pdets) {
     for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
          t += (i64)gridDim.x * blockDim.x) {
-        const u32 r = runid[t] - 1;   // inclusive scan of flags
-        if (t == 0 || k[t].x != k[t - 1].x || k[t].y != k[t - 1].y) {
-            pdets[2 * (i64)r] = k[t].x;
-            pdets[2 * (i64)r + 1] = k[t].y;
-        }
-        col[perm[t]] = r;
+        const u32 r = runid[t];   // inclusive scan of flags
+        if (t > 0 && r == runid[t - 1]) continue;
+        const ulonglong2 d = det_of(k[t], n_orb);
+        pdets[2 * (i64)(r - 1)] = d.x;
+        pdets[2 * (i64)(r - 1) + 1] = d.y;
     }
 }
 
-// (alpha, beta) <-> alpha << n_orb | beta, for n_orb <= 32.
 __global__ void k_pack_keys(const ulonglong2* k, i64 n, int n_orb, u64* out) {
     for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
          t += (i64)gridDim.x * blockDim.x)
         out[t] = (k[t].x << n_orb) | k[t].y;
 }
 
-__global__ void k_unpack_keys(const u64* p, i64 n, int n_orb, ulonglong2* out) {
-    const u64 lo = n_orb >= 64 ? ~0ull : ((1ull << n_orb) - 1);
+// Row of every key in the sorted order.
+__global__ void k_rows_sorted(const u32* rows, const u32* perm, i64 n, u32* out) {
     for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
          t += (i64)gridDim.x * blockDim.x)
-        out[t] = make_ulonglong2(p[t] >> n_orb, p[t] & lo);
+        out[t] = rows[perm[t]];
+}
+
+__global__ void k_vp_entries(const u32* order, const u32* runid, const u32* perm,
+                             const double* vin, i64 n, u32* col, double* val) {
+    for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
+         t += (i64)gridDim.x * blockDim.x) {
+        const u32 u = order[t];
+        col[t] = runid[u] - 1;
+        val[t] = vin[perm[u]];
+    }
 }
 
 // FP32 copy of every value (streaming, 2 values per thread step).
@@ -299,6 +320,32 @@ void exclusive_scan(const T* in, i64* out, i64 n, cudaStream_t s) {
 
 void ensure_sorted(Csr& m, cudaStream_t s) {
     if (!m.sorted) sort_rows(m, s);
+}
+
+// Columns and values of a V->P block in row order, columns ascending, from
+// its keys in sorted order (perm: their places in row order, runid: their
+// columns + 1).  m holds the row pointers and the values in generation order.
+// The keys are in column order already, so a stable sort of their rows is all
+// it takes: two passes for up to 65,536 rows, where sorting every row by
+// column takes a bitonic network or a pass for each byte of (row, column).
+// 6.63e6 entries of 403 rows 1.54 ms before, 0.30 now.
+void order_vp(const u32* perm, const u32* runid, Csr& m, cudaStream_t s) {
+    const i64 n = m.nnz;
+    m.sorted = true;
+    m.col.alloc(n, s);
+    if (n == 0) return;
+    DBuf<u32> rows(n, s), key(n, s), skey(n, s), order(n, s);
+    prim::rows_of(m.rowptr.p, m.nr, n, rows.p, s);
+    k_rows_sorted<<<grid_for(n), 256, 0, s>>>(rows.p, perm, n, key.p);
+    DNQ_CHECK_LAUNCH();
+    int b = 1;
+    while (b < 32 && ((i64)1 << b) < m.nr) ++b;
+    const int bits[1] = {b};
+    prim::radix_sort<u32, u32>(key.p, skey.p, nullptr, order.p, n, bits, s);
+    DBuf<double> val(n, s);
+    k_vp_entries<<<grid_for(n), 256, 0, s>>>(order.p, runid, perm, m.val.p, n, m.col.p, val.p);
+    DNQ_CHECK_LAUNCH();
+    m.val = std::move(val);
 }
 
 
@@ -582,44 +629,40 @@ void build_ham(dnq_ctx_s* ctx, const u64* V_in, i64 nV, const u64* X_in, i64 nX,
     // n_orb <= 32 both strings are packed into one word, alpha above beta,
     // which keeps the (alpha, beta) order.
     require(nvp < (i64)0xffffffffll, DNQ_ERR_OVERFLOW, "H_VP has more than 2^32 entries");
-    DBuf<ulonglong2> ks(nvp, s);
-    DBuf<u32> perm2(nvp, s);
-    if (nvp) {
-        if (2 * n_orb <= 64) {
-            DBuf<u64> pk(nvp, s), pks(nvp, s);
-            k_pack_keys<<<grid_for(nvp), 256, 0, s>>>(vp_key.p, nvp, n_orb, pk.p);
-            DNQ_CHECK_LAUNCH();
-            const int bits[1] = {2 * n_orb};
-            prim::radix_sort<u64, u32>(pk.p, pks.p, nullptr, perm2.p, nvp, bits, s);
-            k_unpack_keys<<<grid_for(nvp), 256, 0, s>>>(pks.p, nvp, n_orb, ks.p);
-            DNQ_CHECK_LAUNCH();
-        } else {
-            const int bits[2] = {n_orb, n_orb};
-            prim::radix_sort<ulonglong2, u32>(vp_key.p, ks.p, nullptr, perm2.p, nvp, bits, s);
-        }
-    }
-    vp_key.release();
-    DBuf<u32> flag(nvp, s), runid(nvp, s);
-    i64 np = 0;
-    if (nvp) {
-        k_unique_flags<<<grid_for(nvp), 256, 0, s>>>(ks.p, nvp, flag.p);
+    DBuf<u32> perm(nvp, s), runid(nvp, s);
+    auto discover = [&](auto* keys, auto* tag) {   // keys sorted: runs, count, determinants
+        using K = std::remove_pointer_t<decltype(tag)>;
+        DBuf<u32> flag(nvp, s);
+        k_unique_flags<K><<<grid_for(nvp), 256, 0, s>>>(keys, nvp, flag.p);
         DNQ_CHECK_LAUNCH();
         prim::scan_inclusive<u32, u32>(flag.p, runid.p, nvp, s);
         u32 last = 0;
         DNQ_CUDA(cudaMemcpyAsync(&last, runid.p + nvp - 1, 4, cudaMemcpyDeviceToHost, s));
         DNQ_CUDA(cudaStreamSynchronize(s));
-        np = last;
-    }
-    H->n_p = np;
-    H->vp.nc = np;
-    H->dets_p.alloc(2 * np, s);
-    H->vp.col.alloc(nvp, s);
-    if (nvp) {
-        k_unique_scatter<<<grid_for(nvp), 256, 0, s>>>(ks.p, perm2.p, runid.p, nvp,
-                                                       H->dets_p.p, H->vp.col.p);
+        H->n_p = last;
+        H->dets_p.alloc(2 * (i64)last, s);
+        k_unique_dets<K><<<grid_for(nvp), 256, 0, s>>>(keys, runid.p, nvp, n_orb, H->dets_p.p);
         DNQ_CHECK_LAUNCH();
+    };
+    H->n_p = 0;
+    if (nvp && 2 * n_orb <= 64) {
+        DBuf<u64> pk(nvp, s), pks(nvp, s);
+        k_pack_keys<<<grid_for(nvp), 256, 0, s>>>(vp_key.p, nvp, n_orb, pk.p);
+        DNQ_CHECK_LAUNCH();
+        vp_key.release();
+        const int bits[1] = {2 * n_orb};
+        prim::radix_sort<u64, u32>(pk.p, pks.p, nullptr, perm.p, nvp, bits, s);
+        pk.release();
+        discover(pks.p, (u64*)nullptr);
+    } else if (nvp) {
+        DBuf<ulonglong2> ks(nvp, s);
+        const int bits[2] = {n_orb, n_orb};
+        prim::radix_sort<ulonglong2, u32>(vp_key.p, ks.p, nullptr, perm.p, nvp, bits, s);
+        vp_key.release();
+        discover(ks.p, (ulonglong2*)nullptr);
     }
-    sort_rows(H->vp, s);
+    H->vp.nc = H->n_p;
+    order_vp(perm.p, runid.p, H->vp, s);
     T.mark();
     T.fill(H->t_ms);
 }

@@ -27,6 +27,7 @@
 
 namespace dnq {
 void keep_pool(int device);
+void order_vp(const u32* perm, const u32* runid, Csr& m, cudaStream_t s);
 
 namespace {
 
@@ -501,15 +502,10 @@ __global__ void k_key4_flags(const Key4* k, i64 n, u32* flag) {
         flag[t] = neq_prev(k, t) ? 1u : 0u;
 }
 
-__global__ void k_key4_scatter(const Key4* k, const u32* perm, const u32* runid, i64 n, u64* pdets,
-                               u32* col) {
+__global__ void k_key4_dets(const Key4* k, const u32* runid, i64 n, Key4* pdets) {
     for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
-         t += (i64)gridDim.x * blockDim.x) {
-        const u32 r = runid[t] - 1;
-        if (neq_prev(k, t))
-            for (int q = 0; q < 4; ++q) pdets[4 * (i64)r + q] = k[t].w[q];
-        col[perm[t]] = r;
-    }
+         t += (i64)gridDim.x * blockDim.x)
+        if (t == 0 || runid[t] != runid[t - 1]) pdets[runid[t] - 1] = k[t];
 }
 
 int blocks(i64 n) {
@@ -701,14 +697,12 @@ void wide_build(dnq_ctx_s* ctx, const u64* V_in, i64 n, const double* psi_in, in
     H->vp.nnz = nvp;
     H->vp.rowptr = std::move(offp);
     H->vp.val = std::move(vpv);
-    H->vp.col.alloc(nvp, s);
     H->dets_p.alloc(4 * np, s);
     if (nvp) {
-        k_key4_scatter<<<blocks(nvp), 256, 0, s>>>(ks.p, perm2.p, runid.p, nvp, (u64*)H->dets_p.p,
-                                                   H->vp.col.p);
+        k_key4_dets<<<blocks(nvp), 256, 0, s>>>(ks.p, runid.p, nvp, (Key4*)H->dets_p.p);
         DNQ_CHECK_LAUNCH();
     }
-    sort_rows(H->vp, s);
+    order_vp(perm2.p, runid.p, H->vp, s);
     DNQ_CUDA(cudaStreamSynchronize(s));
 }
 
