@@ -27,7 +27,10 @@
 //     lanes (a pass moves 2 (key + 4) bytes per key; unordered stores cost it
 //     twice that in partial sectors).
 // Equal digits keep their input order, so the passes compose into a stable
-// sort.  Measured per pass, 4.35e6 (u64, u32) pairs: SORTTIMES.
+// sort.  Measured: a pass over 4.35e6 (u64, u32)
+// pairs 78 us before, 61 now (the scatter 45 -> 38); 2,241 keys of 26 bits 90 us
+// in 30 launches before, 13.5 in one now; 4.2e6 keys of 256 bits, 200 of them
+// significant, 3.3 ms before, 1.9 now.
 //
 // Scan: three phases over tiles of 2048 items (tile sums, one-block scan of
 // the tile sums, tile scans from their offsets), or one block that carries its
