@@ -29,10 +29,13 @@ namespace {
 
 constexpr int kWarpsPerBlock = 8;
 
+template <bool N32>   // at most 32 orbitals
 __global__ void k_diag(CtxView C, const u64* dets, i64 n, double* out) {
     for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
-         t += (i64)gridDim.x * blockDim.x)
-        out[t] = diag_elem(C, dets[2 * t], dets[2 * t + 1]);
+         t += (i64)gridDim.x * blockDim.x) {
+        const u64 a = dets[2 * t], b = dets[2 * t + 1];
+        out[t] = N32 ? diag_elem32(C, (u32)a, (u32)b) : diag_elem(C, a, b);
+    }
 }
 
 __global__ void k_check_orbitals(const u64* dets, i64 n, int n_orb,
@@ -411,7 +414,8 @@ void check_orbitals(const u64* d, i64 n, int n_orb, cudaStream_t s) {
 
 void launch_diag(const dnq_ctx_s* c, const u64* d, i64 n, double* out, cudaStream_t s) {
     if (n == 0) return;
-    k_diag<<<grid_for(n, 128), 128, 0, s>>>(c->view(), d, n, out);
+    (c->n <= 32 ? k_diag<true> : k_diag<false>)<<<grid_for(n, 128), 128, 0, s>>>(c->view(), d, n,
+                                                                                out);
     DNQ_CHECK_LAUNCH();
 }
 

@@ -65,6 +65,38 @@ __device__ __forceinline__ void load_row(WarpRow& R, u64 a, u64 b, int n_orb) {
     __syncwarp();
 }
 
+// diag_elem for at most 32 orbitals, without the list of orbitals (which lies in
+// local memory): strings with orbital 0 in the highest bit, so an orbital is one
+// count of leading zeros.  Chosen at the launch, not here: a kernel that holds
+// both forms has the registers of both (k_pt2_runs 794 us so, 871 with a branch,
+// 1,010 with the list; k_diag at 1e6 dets of 30 orbitals 212 with the list, 176
+// so).
+__device__ __forceinline__ double diag_elem32(const CtxView& C, u32 a, u32 b) {
+    const u32 ra = __brev(a), rb = __brev(b);
+    auto sum = [](double e, const double* t, int stride, u32 x) {
+        while (x) {
+            const int o = __clz(x);
+            x &= ~(0x80000000u >> o);
+            e += __ldg(&t[o * stride]);
+        }
+        return e;
+    };
+    const double one = sum(sum(0.0, C.h1, C.n + 1, ra), C.h1, C.n + 1, rb);
+    double two = 0.0;
+    for (u32 x = ra; x;) {
+        const int p = __clz(x);
+        x &= ~(0x80000000u >> p);
+        two = sum(two, C.dss + p * C.n, 1, ra & ~(0xffffffffu >> p));
+    }
+    for (u32 x = rb; x;) {
+        const int p = __clz(x);
+        x &= ~(0x80000000u >> p);
+        two = sum(two, C.dos + p * C.n, 1, ra);
+        two = sum(two, C.dss + p * C.n, 1, rb & ~(0xffffffffu >> p));
+    }
+    return one + two;
+}
+
 // <bra|H|bra> with the reference's order: one-body over alpha then beta
 // occupied orbitals, then sum_{x>y} <occ_x occ_y||occ_x occ_y>
 // (ham_eval.cpp:53-86).  Serial per thread so the rounding matches.

@@ -366,6 +366,7 @@ struct Pt2Params {
     const u64* V;
     i64 n;
     int n_orb;
+    int key_bits;        // orbitals of the integrals: a double may leave n_orb
     DetMapView mapV;
     const double* coeff;
     double eps1, cut_floor;
@@ -374,12 +375,37 @@ struct Pt2Params {
     int* next_row;
     u32* cnt;
     const i64* off;
-    ulonglong2* keys;
+    void* keys;      // Pt2Key<packed>::type
     double* vals;
 };
 
-template <bool FILL>
+// A determinant as a sort key; PACKED (integrals of at most 32 orbitals): both
+// strings in one word, so the sort moves half the bytes and needs no pass that
+// packs.
+template <bool PACKED>
+struct Pt2Key {
+    using type = u64;
+    static __device__ __forceinline__ u64 make(u64 a, u64 b, int w) { return a << w | b; }
+    static __device__ __forceinline__ bool same(u64 x, u64 y) { return x == y; }
+    static __device__ __forceinline__ ulonglong2 dets(u64 k, int w) {
+        return make_ulonglong2(k >> w, k & ((1ull << w) - 1));
+    }
+};
+template <>
+struct Pt2Key<false> {
+    using type = ulonglong2;
+    static __device__ __forceinline__ ulonglong2 make(u64 a, u64 b, int) {
+        return make_ulonglong2(a, b);
+    }
+    static __device__ __forceinline__ bool same(ulonglong2 x, ulonglong2 y) {
+        return x.x == y.x && x.y == y.y;
+    }
+    static __device__ __forceinline__ ulonglong2 dets(ulonglong2 k, int) { return k; }
+};
+
+template <bool FILL, bool PACKED>
 struct Pt2Sink {
+    using Key = Pt2Key<PACKED>;
     const Pt2Params& P;
     double ci;
     u32 c = 0;
@@ -395,14 +421,14 @@ struct Pt2Sink {
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         if (keep) {
             const i64 at = wpos + __popc(m & lanemask_lt());
-            P.keys[at] = make_ulonglong2(x.a, x.b);
+            static_cast<typename Key::type*>(P.keys)[at] = Key::make(x.a, x.b, P.key_bits);
             P.vals[at] = x.h * ci;
         }
         wpos += __popc(m);
     }
 };
 
-template <bool FILL>
+template <bool FILL, bool PACKED>
 __global__ void __launch_bounds__(kW * 32) k_pt2ext(Pt2Params P) {
     __shared__ WarpRow rows[kW];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -417,7 +443,7 @@ __global__ void __launch_bounds__(kW * 32) k_pt2ext(Pt2Params P) {
             continue;
         }
         load_row(R, P.V[2 * (i64)r], P.V[2 * (i64)r + 1], P.n_orb);
-        Pt2Sink<FILL> sink(P, ci);
+        Pt2Sink<FILL, PACKED> sink(P, ci);
         if (FILL) sink.wpos = P.off[unit];
         if (P.use_hb) {
             const double tau = P.eps1 / fmax(fabs(ci), kAmpDelta);   // :368-372
@@ -441,29 +467,69 @@ __device__ __forceinline__ void tsum2(double a, double b, double& s, double& e) 
 
 // Per unique key: v_a = sum of its contributions (compensated), then
 // v_a^2 / (e_ref - H_aa) with the reference's denominator guard.
-__global__ void k_pt2_runs(CtxView C, const ulonglong2* k, const double* v, i64 n,
-                           double e_ref, double* part, unsigned long long* nuniq) {
+//
+// Bound: the diagonal elements' table reads (L1).  Only the first entry of a
+// run has one, so a warp lists the heads of a tile first and then takes a
+// head per lane; a thread per entry left most lanes waiting for the few
+// heads of their warp.  The contributions stay where they were written and are
+// read through the sorted positions (at), which saves the pass that gathers
+// them.  Measured, 17.9e6 contributions to 5.3e6 determinants of 20 orbitals and
+// 16 electrons: 2.42 ms a thread per entry, 0.84 with heads listed, 0.79 with the
+// gather moved here (it took 0.38 ms, packing the keys 0.09).
+constexpr int kRunTile = 512;
+template <bool PACKED>
+__global__ void __launch_bounds__(256) k_pt2_runs(CtxView C,
+                                                  const typename Pt2Key<PACKED>::type* k,
+                                                  const double* v, const u32* at_of, i64 n,
+                                                  int key_bits, double e_ref, double* part,
+                                                  unsigned long long* nuniq) {
+    using Key = Pt2Key<PACKED>;
+    __shared__ u16 heads_of[8][kRunTile + 1];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    u16* head = heads_of[w];
     double s = 0.0, c = 0.0;
     unsigned long long cnt = 0;
-    for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
-         t += (i64)gridDim.x * blockDim.x) {
-        if (!(t == 0 || k[t].x != k[t - 1].x || k[t].y != k[t - 1].y)) continue;
-        double vs = v[t], vc = 0.0;
-        for (i64 u = t + 1; u < n && k[u].x == k[t].x && k[u].y == k[t].y; ++u) {
-            double s2, e;
-            tsum2(vs, v[u], s2, e);
-            vs = s2;
-            vc += e;
+    for (i64 base = (blockIdx.x * (i64)8 + w) * kRunTile; base < n;
+         base += (i64)gridDim.x * 8 * kRunTile) {
+        const int m = (int)min((i64)kRunTile, n - base);
+        int heads = 0;
+        for (int x = lane; x - lane < m; x += 32) {
+            const i64 t = base + x;
+            const bool h = x < m && (t == 0 || !Key::same(k[t], k[t - 1]));
+            const unsigned b = __ballot_sync(0xffffffffu, h);
+            if (h) head[heads + __popc(b & lanemask_lt())] = (u16)x;
+            heads += __popc(b);
         }
-        const double va = vs + vc;
-        const double haa = diag_elem(C, k[t].x, k[t].y);
-        double den = e_ref - haa;
-        if (fabs(den) < 1e-15) den = den >= 0.0 ? 1e-15 : -1e-15;
-        double s2, e;
-        tsum2(s, (va * va) / den, s2, e);
-        s = s2;
-        c += e;
-        ++cnt;
+        if (lane == 0) head[heads] = (u16)m;
+        __syncwarp();
+        for (int x = lane; x < heads; x += 32) {
+            const i64 t = base + head[x];
+            i64 u = t + 1;
+            const i64 end = base + head[x + 1];
+            double vs = v[at_of[t]], vc = 0.0;
+            auto take = [&] {
+                double s2, e;
+                tsum2(vs, v[at_of[u]], s2, e);
+                vs = s2;
+                vc += e;
+            };
+            const auto key = k[t];
+            for (; u < end; ++u) take();
+            if (x + 1 == heads)   // the tile's last run may go on
+                for (; u < n && Key::same(k[u], key); ++u) take();
+            const double va = vs + vc;
+            const ulonglong2 d = Key::dets(key, key_bits);
+            const double haa =
+                PACKED ? diag_elem32(C, (u32)d.x, (u32)d.y) : diag_elem(C, d.x, d.y);
+            double den = e_ref - haa;
+            if (fabs(den) < 1e-15) den = den >= 0.0 ? 1e-15 : -1e-15;
+            double s2, e;
+            tsum2(s, (va * va) / den, s2, e);
+            s = s2;
+            c += e;
+            ++cnt;
+        }
+        __syncwarp();
     }
     for (int o = 16; o; o >>= 1) {
         const double os = __shfl_xor_sync(0xffffffffu, s, o);
@@ -669,25 +735,16 @@ void local_connections(dnq_ctx_s* ctx, const u64* Vd, i64 n, int n_orb, bool use
     DNQ_CUDA(cudaStreamSynchronize(s));
 }
 
-void pt2(dnq_ctx_s* ctx, const u64* Vd, i64 n, const double* cd, int n_orb, double e_ref,
-         bool use_hb, double eps1, cudaStream_t s, double* out3) {
-    // internal part: full enumeration inside V (local_conn.cpp:303-338)
-    DBuf<double> sigma(n, s), diag(n, s);
-    contract_energy(ctx, Vd, n, cd, n_orb, false, eps1, sigma.p, s);
-    launch_diag(ctx, Vd, n, diag.p, s);
-    const int nb = 4 * sm_count(ctx->device);
-    DBuf<double> part(2 * (i64)nb * 8, s);
-    k_pt2_internal<<<nb, 256, 0, s>>>(sigma.p, cd, diag.p, n, e_ref, part.p);
-    DNQ_CHECK_LAUNCH();
-    out3[0] = sum_parts(part, (i64)nb * 8, s);
-    // external part (:340-415)
+template <bool PACKED>
+void pt2_external(dnq_ctx_s* ctx, const u64* Vd, i64 n, const double* cd, int n_orb, double e_ref,
+                  bool use_hb, double eps1, cudaStream_t s, double* out3) {
     DetMap mapV;
     build_detmap(mapV, Vd, n, false, s);
     DBuf<i64> plen(ctx->tab.n_rows, s);
     k_plen<<<gsz(ctx->tab.n_rows), 256, 0, s>>>(ctx->view().tab, ctx->tab.n_rows,
                                                  full_cutoff(), plen.p);
     DNQ_CHECK_LAUNCH();
-    const int grid = grid_of((const void*)k_pt2ext<false>, ctx->device, kW * 32);
+    const int grid = grid_of((const void*)k_pt2ext<false, PACKED>, ctx->device, kW * 32);
     const int parts = row_parts(n, (i64)grid * kW, n_orb);
     const i64 units = n * parts;
     DBuf<int> next(1, s);
@@ -700,6 +757,7 @@ void pt2(dnq_ctx_s* ctx, const u64* Vd, i64 n, const double* cd, int n_orb, doub
     P.V = Vd;
     P.n = n;
     P.n_orb = n_orb;
+    P.key_bits = ctx->n;
     P.mapV = mapV.view();
     P.coeff = cd;
     P.eps1 = eps1;
@@ -709,35 +767,58 @@ void pt2(dnq_ctx_s* ctx, const u64* Vd, i64 n, const double* cd, int n_orb, doub
     P.next_row = next.p;
     P.cnt = cnt.p;
     DNQ_CUDA(cudaMemsetAsync(next.p, 0, 4, s));
-    k_pt2ext<false><<<grid, kW * 32, 0, s>>>(P);
+    k_pt2ext<false, PACKED><<<grid, kW * 32, 0, s>>>(P);
     DNQ_CHECK_LAUNCH();
     scan_ex(cnt.p, off.p, units + 1, s);
     const i64 tot = rd(off.p + units, s);
-    DBuf<ulonglong2> keys(tot, s), ks(tot, s);
-    DBuf<double> vals(tot, s), vs(tot, s);
+    using Key = typename Pt2Key<PACKED>::type;
+    DBuf<Key> keys(tot, s), ks(tot, s);
+    DBuf<double> vals(tot, s);
+    DBuf<u32> at(tot, s);
     P.off = off.p;
     P.keys = keys.p;
     P.vals = vals.p;
     DNQ_CUDA(cudaMemsetAsync(next.p, 0, 4, s));
-    k_pt2ext<true><<<grid, kW * 32, 0, s>>>(P);
+    k_pt2ext<true, PACKED><<<grid, kW * 32, 0, s>>>(P);
     DNQ_CHECK_LAUNCH();
     out3[1] = 0.0;
     out3[2] = 0.0;
     if (tot == 0) return;
     {
-        const int bits[2] = {n_orb, n_orb};
-        prim::radix_sort<ulonglong2, double>(keys.p, ks.p, vals.p, vs.p, tot, bits, s);
+        const int bits[2] = {PACKED ? 2 * ctx->n : ctx->n, ctx->n};
+        prim::radix_sort<Key, u32>(keys.p, ks.p, nullptr, at.p, tot, bits, s);
+        keys.release();
     }
     DBuf<unsigned long long> nu(1, s);
     DNQ_CUDA(cudaMemsetAsync(nu.p, 0, 8, s));
+    const int nb = grid_of((const void*)k_pt2_runs<PACKED>, ctx->device, 256);
     DBuf<double> part2(2 * (i64)nb * 8, s);
-    k_pt2_runs<<<nb, 256, 0, s>>>(ctx->view(), ks.p, vs.p, tot, e_ref, part2.p, nu.p);
+    k_pt2_runs<PACKED><<<nb, 256, 0, s>>>(ctx->view(), ks.p, vals.p, at.p, tot, ctx->n, e_ref,
+                                          part2.p, nu.p);
     DNQ_CHECK_LAUNCH();
     out3[1] = sum_parts(part2, (i64)nb * 8, s);
     unsigned long long h = 0;
     DNQ_CUDA(cudaMemcpyAsync(&h, nu.p, 8, cudaMemcpyDeviceToHost, s));
     DNQ_CUDA(cudaStreamSynchronize(s));
     out3[2] = (double)h;
+}
+
+void pt2(dnq_ctx_s* ctx, const u64* Vd, i64 n, const double* cd, int n_orb, double e_ref,
+         bool use_hb, double eps1, cudaStream_t s, double* out3) {
+    // internal part: full enumeration inside V (local_conn.cpp:303-338)
+    DBuf<double> sigma(n, s), diag(n, s);
+    contract_energy(ctx, Vd, n, cd, n_orb, false, eps1, sigma.p, s);
+    launch_diag(ctx, Vd, n, diag.p, s);
+    const int nb = 4 * sm_count(ctx->device);
+    DBuf<double> part(2 * (i64)nb * 8, s);
+    k_pt2_internal<<<nb, 256, 0, s>>>(sigma.p, cd, diag.p, n, e_ref, part.p);
+    DNQ_CHECK_LAUNCH();
+    out3[0] = sum_parts(part, (i64)nb * 8, s);
+    // external part (:340-415)
+    if (ctx->n <= 32)
+        pt2_external<true>(ctx, Vd, n, cd, n_orb, e_ref, use_hb, eps1, s, out3);
+    else
+        pt2_external<false>(ctx, Vd, n, cd, n_orb, e_ref, use_hb, eps1, s, out3);
 }
 
 }  // namespace dnq
