@@ -810,7 +810,7 @@ __device__ __forceinline__ u32 exc_tag(u32 kind, W x, int h, int p) {
 
 // Bound: instructions and the latency of the gathers (string, index,
 // integral): 327 instructions per 32 members of a 30-orbital space with 64-bit
-// strings, index and phase arithmetic.  k_vv_eval at 1e6 rows 3.80 -> 2.77 ms.
+// strings, index and phase arithmetic.  k_vv_eval at 1e6 rows 3.80 -> 2.8 to 3.0 ms.
 // AHEAD: singles read their integrals ahead of the additions.
 template <class W, bool AHEAD = true>
 __device__ __forceinline__ Hit eval_hit(const VVParams& P, int r, u64 a, u64 b, double psr,
