@@ -200,8 +200,15 @@ int group_for(const Csr& m) {
     return 4;
 }
 
-// Slots in flight per lane: as many as the average row fills, at most 4.
+// Slots in flight per lane: as many as the average row fills, at most 4.  A
+// block whose rows all run at once takes as long as its longest row (a row
+// connected to most of the space, with the lanes of an average one), so it
+// keeps 4: 10,007 wide rows of which one is full 449 us with 1, 168 with 4 (a
+// launch; 2,241 rows with a full one 12.8 us with 2, 10.2 with 4).  Larger blocks
+// are bound by the gathers, where 4 slots would cost a third of the warps.
+constexpr i64 kOneRound = 2 * 148 * 256;   // lanes that run at once with 4 slots
 int unroll_for(const Csr& m, int G) {
+    if (m.nr * G <= kOneRound) return 4;
     const double avg = m.nr ? (double)m.nnz / (double)m.nr : 0.0;
     const double slots = avg / (4.0 * G);
     if (slots >= 4) return 4;
