@@ -99,8 +99,10 @@ __device__ __forceinline__ bool lu_rows(T (&a)[N], int n, int r, int gbase, int&
         const int src = gbase + (who ? __ffs(who) - 1 : 0);
         const bool is_piv = gbase + r == src && who;
         par ^= br != k;
+        // no row is moved in a column without a usable value (br == n), so the
+        // positions stay a permutation of the n rows
         if (is_piv) pos = k;
-        else if (pos == k) pos = br;
+        else if (pos == k && br < n) pos = br;
         const T p = __shfl_sync(0xffffffffu, a[k], src);
         if (r == k) piv = p;
         const bool below = r < n && pos > k;
@@ -182,7 +184,8 @@ k_slogdet_grad_rows(const T* A, const T* cot, i64 B, int n, T* grad) {
         T piv;
         const bool ok = lu_rows<T, N>(a, n, r, gbase, pos, piv, par);
         __syncwarp();
-        if (have) {   // the factors, rows where the exchanges put them
+        const bool solve = have && ok;   // a singular matrix' gradient is 0
+        if (solve) {   // the factors, rows where the exchanges put them
 #pragma unroll
             for (int j = 0; j < N; ++j)
                 if (j < n) S[m * nn + pos * n + j] = a[j];
@@ -191,7 +194,7 @@ k_slogdet_grad_rows(const T* A, const T* cot, i64 B, int n, T* grad) {
         // column r of Y: row r of I stands at row pos
         T y[N] = {};
         const T* F = S + m * nn;
-        if (have) {
+        if (solve) {
             static_for<N>([&](auto row) {   // L z = e (unit diagonal)
                 constexpr int i = decltype(row)::value;
                 if (i >= n) return;
