@@ -26,6 +26,7 @@ namespace dnq {
 // Per-warp occupancy lists, in shared memory.
 struct WarpRow {
     u64 a, b;                 // bra alpha / beta masks
+    u64 fulla, fullb;         // no place for a particle: occupied, or not among the n_orb
     int na, nb, nva, nvb, ne;
     u8 occ[128];              // spin-orbitals: 2p (alpha asc) then 2p+1 (beta asc)
     u8 occa[64], occb[64], vira[64], virb[64];
@@ -56,6 +57,8 @@ __device__ __forceinline__ void load_row(WarpRow& R, u64 a, u64 b, int n_orb) {
     if (lane == 0) {
         R.a = a;
         R.b = b;
+        R.fulla = a | ~all;
+        R.fullb = b | ~all;
         R.na = na;
         R.nb = nb;
         R.ne = na + nb;
@@ -297,6 +300,8 @@ __device__ __forceinline__ void pair_of(int p, int& x, int& y) {
 }
 
 // Doubles over the occupied pairs [p_lo, p_hi) (x ascending, y < x ascending).
+// The table lists particles among all orbitals of the integrals; one past n_orb
+// is no candidate (ham_utils.cpp:470-479).
 // The table rows of 32 pairs are looked up at once, a pair per lane, and the
 // prefixes of a cut of the row's own searched side by side: one pair after
 // the other, a warp waits several L2 reads for each, most of them for an empty
@@ -355,9 +360,9 @@ __device__ __forceinline__ void enumerate_pairs(const CtxView& C, const WarpRow&
                     const double v = __ldg(&C.tab.v[lo + e]);
                     const int A = ab & 0xff, B = ab >> 8;
                     const u64 ma = 1ull << (A >> 1), mb = 1ull << (B >> 1);
-                    const bool occA = ((A & 1) ? R.b : R.a) & ma;
-                    const bool occB = ((B & 1) ? R.b : R.a) & mb;
-                    if (occA || occB) {
+                    const bool noA = ((A & 1) ? R.fullb : R.fulla) & ma;
+                    const bool noB = ((B & 1) ? R.fullb : R.fulla) & mb;
+                    if (noA || noB) {
                         c.valid = false;
                     } else {
                         c.a = ha | ((A & 1) ? 0ull : ma) | ((B & 1) ? 0ull : mb);

@@ -366,7 +366,6 @@ struct Pt2Params {
     const u64* V;
     i64 n;
     int n_orb;
-    int key_bits;        // orbitals of the integrals: a double may leave n_orb
     DetMapView mapV;
     const double* coeff;
     double eps1, cut_floor;
@@ -379,7 +378,7 @@ struct Pt2Params {
     double* vals;
 };
 
-// A determinant as a sort key; PACKED (integrals of at most 32 orbitals): both
+// A determinant as a sort key; PACKED (at most 32 orbitals): both
 // strings in one word, so the sort moves half the bytes and needs no pass that
 // packs.
 template <bool PACKED>
@@ -421,7 +420,7 @@ struct Pt2Sink {
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         if (keep) {
             const i64 at = wpos + __popc(m & lanemask_lt());
-            static_cast<typename Key::type*>(P.keys)[at] = Key::make(x.a, x.b, P.key_bits);
+            static_cast<typename Key::type*>(P.keys)[at] = Key::make(x.a, x.b, P.n_orb);
             P.vals[at] = x.h * ci;
         }
         wpos += __popc(m);
@@ -481,7 +480,7 @@ template <bool PACKED>
 __global__ void __launch_bounds__(256) k_pt2_runs(CtxView C,
                                                   const typename Pt2Key<PACKED>::type* k,
                                                   const double* v, const u32* at_of, i64 n,
-                                                  int key_bits, double e_ref, double* part,
+                                                  int n_orb, double e_ref, double* part,
                                                   unsigned long long* nuniq) {
     using Key = Pt2Key<PACKED>;
     __shared__ u16 heads_of[8][kRunTile + 1];
@@ -518,7 +517,7 @@ __global__ void __launch_bounds__(256) k_pt2_runs(CtxView C,
             if (x + 1 == heads)   // the tile's last run may go on
                 for (; u < n && Key::same(k[u], key); ++u) take();
             const double va = vs + vc;
-            const ulonglong2 d = Key::dets(key, key_bits);
+            const ulonglong2 d = Key::dets(key, n_orb);
             const double haa =
                 PACKED ? diag_elem32(C, (u32)d.x, (u32)d.y) : diag_elem(C, d.x, d.y);
             double den = e_ref - haa;
@@ -757,7 +756,6 @@ void pt2_external(dnq_ctx_s* ctx, const u64* Vd, i64 n, const double* cd, int n_
     P.V = Vd;
     P.n = n;
     P.n_orb = n_orb;
-    P.key_bits = ctx->n;
     P.mapV = mapV.view();
     P.coeff = cd;
     P.eps1 = eps1;
@@ -785,7 +783,7 @@ void pt2_external(dnq_ctx_s* ctx, const u64* Vd, i64 n, const double* cd, int n_
     out3[2] = 0.0;
     if (tot == 0) return;
     {
-        const int bits[2] = {PACKED ? 2 * ctx->n : ctx->n, ctx->n};
+        const int bits[2] = {PACKED ? 2 * n_orb : n_orb, n_orb};
         prim::radix_sort<Key, u32>(keys.p, ks.p, nullptr, at.p, tot, bits, s);
         keys.release();
     }
@@ -793,7 +791,7 @@ void pt2_external(dnq_ctx_s* ctx, const u64* Vd, i64 n, const double* cd, int n_
     DNQ_CUDA(cudaMemsetAsync(nu.p, 0, 8, s));
     const int nb = grid_of((const void*)k_pt2_runs<PACKED>, ctx->device, 256);
     DBuf<double> part2(2 * (i64)nb * 8, s);
-    k_pt2_runs<PACKED><<<nb, 256, 0, s>>>(ctx->view(), ks.p, vals.p, at.p, tot, ctx->n, e_ref,
+    k_pt2_runs<PACKED><<<nb, 256, 0, s>>>(ctx->view(), ks.p, vals.p, at.p, tot, n_orb, e_ref,
                                           part2.p, nu.p);
     DNQ_CHECK_LAUNCH();
     out3[1] = sum_parts(part2, (i64)nb * 8, s);
@@ -815,7 +813,7 @@ void pt2(dnq_ctx_s* ctx, const u64* Vd, i64 n, const double* cd, int n_orb, doub
     DNQ_CHECK_LAUNCH();
     out3[0] = sum_parts(part, (i64)nb * 8, s);
     // external part (:340-415)
-    if (ctx->n <= 32)
+    if (n_orb <= 32)
         pt2_external<true>(ctx, Vd, n, cd, n_orb, e_ref, use_hb, eps1, s, out3);
     else
         pt2_external<false>(ctx, Vd, n, cd, n_orb, e_ref, use_hb, eps1, s, out3);
