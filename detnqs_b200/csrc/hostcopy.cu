@@ -2,11 +2,11 @@
 
 #include "hostcopy.cuh"
 
-#include <atomic>
 #include <algorithm>
+#include <atomic>
+#include <condition_variable>
 #include <cstring>
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 namespace dnq {
@@ -103,54 +103,84 @@ void HostCopies::run() {
         DNQ_CUDA(cudaStreamSynchronize(s_));
         return;
     }
-    int dev = 0;
-    std::atomic<int> failed{(int)cudaGetDevice(&dev)};
+    // All copies are issued by this thread: a stream handle need not name the
+    // same stream in another one (cudaStreamPerThread).  Chunk i fills slot
+    // i % ns once chunk i - ns is copied out of it; the workers take the chunks
+    // in order, wait for their events and copy on.
     const unsigned cores = std::thread::hardware_concurrency();
     const int nw = (int)std::max<size_t>(
         1, std::min<size_t>({(size_t)kWorkers, (size_t)(cores > 1 ? cores / 2 : 1), todo.size() / 2}));
-    // Worker w copies chunks w, w + nw, ...: the next one fills a slot on the
-    // stream while the last one is copied out of the other.
+    const size_t ns = 2 * (size_t)nw;
+    cudaEvent_t ev[2 * kWorkers] = {};
+    std::mutex mu;
+    std::condition_variable filled, freed;
+    size_t issued = 0;               // chunks issued
+    size_t out[2 * kWorkers] = {};   // per slot: chunks copied out of it
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    bool stop = false;
+    cudaError_t failed = cudaSuccess;
     std::atomic<size_t> next{0};
-    auto work = [&](int w) noexcept {
-        cudaEvent_t ev[2] = {};
-        cudaError_t e = cudaSetDevice(dev);
-        for (auto& x : ev)
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
-        char* slot[2] = {slots + 2 * w * kChunk, slots + (2 * w + 1) * kChunk};
-        const Piece* held[2] = {};
-        int k = 0;
+    auto work = [&]() noexcept {
+        cudaError_t err = cudaSetDevice(dev);
         for (;;) {
-            const size_t i = e == cudaSuccess && !failed.load() ? next++ : todo.size();
-            if (i < todo.size()) {
-                held[k] = &todo[i];
-                e = cudaMemcpyAsync(slot[k], todo[i].src, todo[i].n, cudaMemcpyDeviceToHost, s_);
-                if (e == cudaSuccess) e = cudaEventRecord(ev[k], s_);
-            } else {
-                held[k] = nullptr;
+            const size_t i = next++;
+            if (i >= todo.size()) break;
+            {
+                std::unique_lock<std::mutex> lk(mu);
+                if (err == cudaSuccess) filled.wait(lk, [&] { return issued > i || stop; });
+                if (err != cudaSuccess || issued <= i) break;
             }
-            k ^= 1;
-            if (held[k] && e == cudaSuccess) {
-                e = cudaEventSynchronize(ev[k]);
-                if (e == cudaSuccess) std::memcpy(held[k]->dst, slot[k], held[k]->n);
-            }
-            if (e != cudaSuccess || (!held[0] && !held[1])) break;
-            held[k] = nullptr;
+            const size_t q = i % ns;
+            err = cudaEventSynchronize(ev[q]);
+            if (err == cudaSuccess) std::memcpy(todo[i].dst, slots + q * kChunk, todo[i].n);
+            std::lock_guard<std::mutex> lk(mu);
+            if (err != cudaSuccess) break;
+            ++out[q];
+            freed.notify_one();
         }
-        if (e != cudaSuccess) failed = (int)e;
-        for (auto& x : ev)
-            if (x) cudaEventDestroy(x);
+        if (err != cudaSuccess) {
+            std::lock_guard<std::mutex> lk(mu);
+            failed = err;
+            stop = true;
+            filled.notify_all();
+            freed.notify_one();
+        }
     };
+    for (size_t q = 0; q < ns && e == cudaSuccess; ++q)
+        e = cudaEventCreateWithFlags(&ev[q], cudaEventDisableTiming);
     std::vector<std::thread> team;
     try {
-        team.reserve(nw - 1);
-        for (int w = 1; w < nw; ++w) team.emplace_back(work, w);
+        team.reserve(nw);
+        while (e == cudaSuccess && (int)team.size() < nw) team.emplace_back(work);
     } catch (const std::exception&) {   // fewer threads: the chunks are shared out as they go
     }
-    work(0);
+    const bool alone = team.empty();   // no thread at all: plain copies
+    for (size_t i = 0; i < todo.size() && e == cudaSuccess; ++i) {
+        if (alone) {
+            e = cudaMemcpyAsync(todo[i].dst, todo[i].src, todo[i].n, cudaMemcpyDeviceToHost, s_);
+            continue;
+        }
+        const size_t q = i % ns;
+        {
+            std::unique_lock<std::mutex> lk(mu);
+            freed.wait(lk, [&] { return out[q] == i / ns || stop; });
+            if (stop) break;
+        }
+        e = cudaMemcpyAsync(slots + q * kChunk, todo[i].src, todo[i].n, cudaMemcpyDeviceToHost, s_);
+        if (e == cudaSuccess) e = cudaEventRecord(ev[q], s_);
+        std::lock_guard<std::mutex> lk(mu);
+        if (e == cudaSuccess) issued = i + 1;
+        else stop = true;
+        filled.notify_all();
+    }
     for (auto& t : team) t.join();
     const cudaError_t done = cudaStreamSynchronize(s_);   // no copy into a slot is left
+    for (auto& x : ev)
+        if (x) cudaEventDestroy(x);
     pool().give(slots);
-    DNQ_CUDA((cudaError_t)failed.load());
+    DNQ_CUDA(e);
+    DNQ_CUDA(failed);
     DNQ_CUDA(done);
 }
 

@@ -3,9 +3,10 @@
 // The driver copies to pageable memory through one staging thread, which also
 // takes the page faults of a fresh result array: 5 GB/s measured for the 220 MB
 // of blocks of a 403-row proxy build.  Copies of kHostCopyMin bytes or more
-// go through page-locked slots instead, each worker thread copying its share
-// of the chunks on (and faulting it in) while the GPU fills its other slot:
-// 106 MB of H_VP in 24 ms before, 5.6 ms now.
+// go through page-locked slots instead: the calling thread, the only one to use
+// the caller's stream, keeps the GPU filling free slots while worker threads
+// copy the chunks on (and fault them in).  106 MB of H_VP in 24 ms before, 5.6 ms
+// now.
 #pragma once
 
 #include <vector>
