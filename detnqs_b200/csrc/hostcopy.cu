@@ -18,26 +18,37 @@ constexpr size_t kChunk = size_t(2) << 20;
 constexpr int kWorkers = 8;                      // at most
 constexpr size_t kSlots = 2 * kWorkers * kChunk;  // 32 MiB: two slots per worker
 constexpr int kKept = 2;                          // slot sets kept for later copies
+// A slot set takes the driver 31 ms to lock and 3.5 to release, as long as the
+// plain copies of about this many bytes take more than the staged ones (111 MB
+// into fresh arrays: 17 to 27 ms plain, 4.2 staged).
+constexpr size_t kWorth = size_t(192) << 20;
 
 struct SlotPool {
     std::mutex mu;
     char* kept[kKept] = {};
+    int made = 0;       // sets there are, kept or in use
     long contexts = 0;
-    char* take() {
-        {
-            std::lock_guard<std::mutex> lk(mu);
-            for (auto& p : kept)
-                if (p) {
-                    char* q = p;
-                    p = nullptr;
-                    return q;
-                }
-        }
+    size_t plain = 0;   // bytes copied the plain way under these contexts
+    // A slot set for a copy of n bytes, or null: the plain copy does it.  A set
+    // is made only where it can be kept, and once the plain copies have cost as
+    // much.
+    char* take(size_t n) {
+        std::lock_guard<std::mutex> lk(mu);
+        for (auto& p : kept)
+            if (p) {
+                char* q = p;
+                p = nullptr;
+                return q;
+            }
+        if (contexts == 0 || made == kKept) return nullptr;
+        plain += n;
+        if (plain < kWorth) return nullptr;
         void* q = nullptr;
         if (cudaHostAlloc(&q, kSlots, cudaHostAllocPortable) != cudaSuccess) {
             (void)cudaGetLastError();
-            return nullptr;   // no page-locked memory: the plain copy does it
+            return nullptr;   // no page-locked memory
         }
+        ++made;
         return static_cast<char*>(q);
     }
     void give(char* q) noexcept {
@@ -49,6 +60,7 @@ struct SlotPool {
                         p = q;
                         return;
                     }
+            --made;
         }
         cudaFreeHost(q);
     }
@@ -72,8 +84,13 @@ void host_slots_drop() noexcept {
     char* old[kKept] = {};
     {
         std::lock_guard<std::mutex> lk(P.mu);
-        if (--P.contexts == 0)
-            for (int k = 0; k < kKept; ++k) std::swap(old[k], P.kept[k]);
+        if (--P.contexts == 0) {
+            for (int k = 0; k < kKept; ++k) {
+                std::swap(old[k], P.kept[k]);
+                if (old[k]) --P.made;
+            }
+            P.plain = 0;
+        }
     }
     for (char* p : old)
         if (p) cudaFreeHost(p);
@@ -96,7 +113,9 @@ void HostCopies::add_bytes(void* dst, const void* src, size_t n) {
 void HostCopies::run() {
     std::vector<Piece> todo;
     todo.swap(pieces_);
-    char* slots = todo.empty() ? nullptr : pool().take();
+    size_t bytes = 0;
+    for (const Piece& p : todo) bytes += p.n;
+    char* slots = todo.empty() ? nullptr : pool().take(bytes);
     if (!slots) {
         for (const Piece& p : todo)
             DNQ_CUDA(cudaMemcpyAsync(p.dst, p.src, p.n, cudaMemcpyDeviceToHost, s_));

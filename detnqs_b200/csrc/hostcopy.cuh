@@ -39,7 +39,8 @@ private:
 };
 
 // Contexts alive: the page-locked slots kept between copies are released with
-// the last of them.
+// the last of them, and none are made without one (locking and releasing them
+// for every copy took get_ham_eff of 2e6 entries from 4.8 to 39 ms).
 void host_slots_hold();
 void host_slots_drop() noexcept;
 struct HostSlots {
