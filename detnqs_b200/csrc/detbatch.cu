@@ -162,7 +162,7 @@ k_det_batch(const u64* dets, i64 B, u64 ref_a, u64 ref_b, int n_orb, int na, int
             for (W x = a; x;) *p++ = take_low(x);
             for (W x = b; x;) *p++ = take_low(x) + n_orb;
         }
-        if (ne) piece_out(o.occ + i0 * ne, ne, buf, ne, cnt, lane);
+        if (ne && na <= n_orb && nb <= n_orb) piece_out(o.occ + i0 * ne, ne, buf, ne, cnt, lane);
         W ha = ra & ~a, hb = rb & ~b, pa = a & ~ra, pb = b & ~rb;
         const int kk = Bits<W>::count(ha) + Bits<W>::count(hb);
         if (on && (flags & (kNeedK | kNeedHp))) o.k[i] = (int8_t)min(kk, 127);
@@ -308,9 +308,12 @@ int dnq_prepare_det_batch(const uint64_t* dets, int64_t B, const uint64_t* ref, 
     DBuf<unsigned long long> err(1, s);
     DNQ_CUDA(cudaMemsetAsync(err.p, 0xff, sizeof(unsigned long long), s));
     BatchOut bo{o_occ.p, o_k.p, o_ph.p, o_h.p, o_p.p, o_m.p, o_hp.p, o_pp.p};
-    // words of a warp's pieces: at most 4 x 32 x 33, 66 KB a block
+    // words of a warp's pieces: at most 32 x 4 x 33, 66 KB a block.  With more
+    // electrons of a spin than orbitals no determinant has a row to stage (the
+    // kernel reports the first)
     const int kc = need_hp ? std::min(kmax, kListCols) : 0;
-    const int piece_words = 32 * std::max(ne | 1, (kc | 1) * (need_pos ? 4 : 2));
+    const int row = n_alpha <= n_orb && n_beta <= n_orb ? ne : 0;
+    const int piece_words = 32 * std::max(row | 1, (kc | 1) * (need_pos ? 4 : 2));
     const size_t smem = (size_t)kFeatWarps * piece_words * sizeof(int32_t);
     auto kern = n_orb <= 32 ? k_det_batch<u32> : k_det_batch<u64>;
     if (smem > 48 * 1024)
