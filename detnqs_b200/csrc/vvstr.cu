@@ -2056,19 +2056,13 @@ void launch_eval_long(int scan, int grid, const Loc& L, const Arena& A, cudaStre
     DNQ_CHECK_LAUNCH();
 }
 
-// Single-pass build of nrows rows of L into M (allocated here).  cap_hint:
-// expected nnz (0 = unknown).  Falls back to the exact two-pass walk when
-// the arena is too small.  With arena_out, M keeps the rows where the build
-// wrote them (arena form: the arena becomes M's storage, no compaction);
-// else they are compacted into a standard CSR.  With dg, the build also
-// writes M.val32 (the FP32 values, diagonal entries zero) and the FP64
-// diagonal into *dg; the two-pass fallback leaves both empty.  Returns the
-// number of member tests.
+// run_vv, for one size of the arena.  look: size it by the free memory (set
+// where that was done).
 template <class Loc>
-i64 run_vv(const Loc& L, i64 nrows, i64 cap_hint, int device, cudaStream_t s, Csr& M,
-           const Options& opt, double* t_gen, double* t_scan, double* t_compact,
-           i64* hits_out = nullptr, int scan = 0, DBuf<double>* dg = nullptr,
-           const u32* order = nullptr, bool arena_out = false) {
+i64 run_vv_with(const Loc& L, i64 nrows, i64 cap_hint, int device, cudaStream_t s, Csr& M,
+                const Options& opt, double* t_gen, double* t_scan, double* t_compact,
+                i64* hits_out, int scan, DBuf<double>* dg, const u32* order, bool arena_out,
+                bool& look) {
     Events<4> ev;
     const int grid = vv_grid<Loc>(device);
     const i64 warps = (i64)grid * kWS;
@@ -2081,10 +2075,12 @@ i64 run_vv(const Loc& L, i64 nrows, i64 cap_hint, int device, cudaStream_t s, Cs
     const bool f32_in_build = arena_out && dg;   // k_vv_eval writes the FP32 copy
     // at most half of the free memory; what the device's pool holds unused (as
     // after an earlier build of this size) needs no look at that, which
-    // takes the driver 70 us, and 0.2-0.8 ms one time in ten
+    // takes the driver 70 us, and 0.2-0.8 ms one time in ten.  Rows that are
+    // compacted need as much again.
     const i64 slot_bytes = f32_in_build ? 16 : 12;
     i64 cap = std::max<i64>(want, chunk);
-    if (pool_unused(device) < cap * slot_bytes) {
+    look = look || pool_unused(device) < cap * slot_bytes * (arena_out ? 1 : 2);
+    if (look) {
         size_t freeb = 0, totb = 0;
         DNQ_CUDA(cudaMemGetInfo(&freeb, &totb));
         cap = std::max<i64>(std::min(want, (i64)freeb / 2 / slot_bytes), chunk);
@@ -2265,6 +2261,34 @@ i64 run_vv(const Loc& L, i64 nrows, i64 cap_hint, int device, cudaStream_t s, Cs
     DNQ_CUDA(cudaEventElapsedTime(&ms, ev[2], ev[3]));
     if (t_compact) *t_compact = ms;
     return (i64)tests;
+}
+
+// Single-pass build of nrows rows of L into M (allocated here).  cap_hint:
+// expected nnz (0 = unknown).  Falls back to the exact two-pass walk when
+// the arena is too small.  With arena_out, M keeps the rows where the build
+// wrote them (arena form: the arena becomes M's storage, no compaction);
+// else they are compacted into a standard CSR.  With dg, the build also
+// writes M.val32 (the FP32 values, diagonal entries zero) and the FP64
+// diagonal into *dg; the two-pass fallback leaves both empty.  Returns the
+// number of member tests.
+template <class Loc>
+i64 run_vv(const Loc& L, i64 nrows, i64 cap_hint, int device, cudaStream_t s, Csr& M,
+           const Options& opt, double* t_gen, double* t_scan, double* t_compact,
+           i64* hits_out = nullptr, int scan = 0, DBuf<double>* dg = nullptr,
+           const u32* order = nullptr, bool arena_out = false) {
+    bool look = opt.arena_cap > 0;   // a given capacity is taken as it is
+    try {
+        return run_vv_with(L, nrows, cap_hint, device, s, M, opt, t_gen, t_scan, t_compact,
+                           hits_out, scan, dg, order, arena_out, look);
+    } catch (const Error& x) {
+        // the pool's unused memory was in pieces, or taken meanwhile: an arena
+        // of half the free memory, and the two-pass walk where that is too small
+        if (look || x.code != DNQ_ERR_OUT_OF_MEMORY) throw;
+    }
+    M = Csr{};
+    look = true;
+    return run_vv_with(L, nrows, cap_hint, device, s, M, opt, t_gen, t_scan, t_compact, hits_out,
+                       scan, dg, order, arena_out, look);
 }
 
 VVParams make_params(dnq_ctx_s* ctx, const u64* V, i64 n, int n_orb, int policy, double eps1,
