@@ -84,7 +84,7 @@ struct SpmvDesc {
     i64 nr, nnz;         // rows; length of col / val (bounds the vector loads)
 };
 // Lanes per row and slots per lane the H.psi kernels use for m.
-void spmv_shape(const Options& o, const Csr& m, int& G, int& U);
+void spmv_shape(const Options& o, const Csr& m, int device, int& G, int& U);
 // One launch over nd descriptors (device array) sharing (G, U, precision).
 void spmv_grouped(const SpmvDesc* d_dev, int nd, i64 max_rows, int G, int U, int precision,
                   int device, cudaStream_t s);

@@ -353,7 +353,7 @@ void launch_group(dnq_server_s* S) {
         ed[k] = EnergyDesc{S->gx.p + o, S->gy.p + o, S->geloc.p + o, f32 ? S->gx32.p + o : nullptr,
                            h->n_v};
         int G = 4, U = 1;
-        spmv_shape(h->opt, h->vv, G, U);
+        spmv_shape(h->opt, h->vv, h->device, G, U);
         SpmvDesc d{};
         d.rp = h->vv.row_start();
         d.re = h->vv.row_end();

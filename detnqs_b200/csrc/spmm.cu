@@ -26,7 +26,7 @@
 
 namespace dnq {
 
-void spmv_shape(const Options& o, const Csr& m, int& G, int& U);
+void spmv_shape(const Options& o, const Csr& m, int device, int& G, int& U);
 void ensure_f32(dnq_ham_s* h, cudaStream_t s);
 
 namespace {
@@ -335,7 +335,7 @@ void spmm_csr(const Csr& m, const float* val32, const double* diag32, const doub
     if (m.nr == 0) return;
     if (G == 0 || U == 0) {
         int g = 0, u = 0;
-        spmv_shape(Options{}, m, g, u);
+        spmv_shape(Options{}, m, dev, g, u);
         if (G == 0) G = g;
         if (U == 0) U = u;
     }

@@ -206,9 +206,9 @@ int group_for(const Csr& m) {
 // keeps 4: 10,007 wide rows of which one is full 449 us with 1, 168 with 4 (a
 // launch; 2,241 rows with a full one 12.8 us with 2, 10.2 with 4).  Larger blocks
 // are bound by the gathers, where 4 slots would cost a third of the warps.
-constexpr i64 kOneRound = 2 * 148 * 256;   // lanes that run at once with 4 slots
-int unroll_for(const Csr& m, int G) {
-    if (m.nr * G <= kOneRound) return 4;
+constexpr i64 kOneRound = 2 * 256;   // lanes of an SM that run at once with 4 slots
+int unroll_for(const Csr& m, int G, int device) {
+    if (m.nr * G <= kOneRound * sm_count(device)) return 4;
     const double avg = m.nr ? (double)m.nnz / (double)m.nr : 0.0;
     const double slots = avg / (4.0 * G);
     if (slots >= 4) return 4;
@@ -256,7 +256,7 @@ void launch_spmv(const Csr& m, const double* x, double* y, const double* yadd, i
                  int device, cudaStream_t s) {
     if (m.nr == 0) return;
     if (G == 0) G = group_for(m);
-    if (U == 0) U = unroll_for(m, G);
+    if (U == 0) U = unroll_for(m, G, device);
     switch (G) {
         case 32: launch_g<32>(U, m, x, y, yadd, precision, x32, val32, diag, device, s); break;
         case 16: launch_g<16>(U, m, x, y, yadd, precision, x32, val32, diag, device, s); break;
@@ -286,9 +286,9 @@ void spmv_block(const dnq_ham_s* h, const Csr& m, const double* x, double* y,
                 h->opt.spmv_unroll, h->device, s);
 }
 
-void spmv_shape(const Options& o, const Csr& m, int& G, int& U) {
+void spmv_shape(const Options& o, const Csr& m, int device, int& G, int& U) {
     G = o.spmv_lanes ? o.spmv_lanes : group_for(m);
-    U = o.spmv_unroll ? o.spmv_unroll : unroll_for(m, G);
+    U = o.spmv_unroll ? o.spmv_unroll : unroll_for(m, G, device);
 }
 
 namespace {
