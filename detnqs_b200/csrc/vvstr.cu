@@ -75,6 +75,7 @@ struct StrIndex {
     DBuf<u32> gid;       // group number of every sorted position
     DBuf<u32> gstart;    // first sorted position of every group, then n
     i64 ngroups = 0;
+    bool mixed = false;  // alpha index: determinants of several electron counts
     DBuf<ulonglong2> slots;
     u64 mask = 0;
     // Presence rows (alpha index only): one bit per beta group for every
@@ -105,14 +106,32 @@ __global__ void k_keys_by(const u64* V, i64 n, int major, ulonglong2* k) {
     }
 }
 
-// dup (optional) is set when two sorted keys are equal: a determinant listed
-// twice.
-__global__ void k_split_sorted(const ulonglong2* k, i64 n, u64* other, unsigned* head, u32* dup) {
+// What the host reads of an index after its first phase: the group count,
+// whether a determinant is listed twice, whether electron counts differ (the
+// string tests count differing orbitals, which then says nothing of the
+// excitation rank), and the group lengths by floor(log2(len - 1)).
+struct IndexProbe {
+    u32 ngroups;
+    u32 dup;
+    u32 mixed;
+    u32 hist[32];
+};
+
+// Neighbours of the sorted order: equal ones are a determinant listed twice,
+// and one with other electron counts shows that the counts are not all the same.
+__device__ __forceinline__ void probe_pair(IndexProbe* probe, u64 a, u64 b, u64 a0, u64 b0) {
+    if (a == a0 && b == b0) probe->dup = 1u;
+    if (__popcll(a) != __popcll(a0) || __popcll(b) != __popcll(b0)) probe->mixed = 1u;
+}
+
+// probe is optional.
+__global__ void k_split_sorted(const ulonglong2* k, i64 n, u64* other, unsigned* head,
+                               IndexProbe* probe) {
     for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
          t += (i64)gridDim.x * blockDim.x) {
         other[t] = k[t].y;
         head[t] = (t == 0 || k[t].x != k[t - 1].x) ? 1u : 0u;
-        if (dup && t > 0 && k[t].x == k[t - 1].x && k[t].y == k[t - 1].y) *dup = 1u;
+        if (probe && t > 0) probe_pair(probe, k[t].x, k[t].y, k[t - 1].x, k[t - 1].y);
     }
 }
 
@@ -158,13 +177,14 @@ __global__ void k_keys_by64(const u64* V, i64 n, int major, u64* k) {
 }
 
 __global__ void k_split_sorted64(const u64* k, i64 n, u64* other, u32* other32, unsigned* head,
-                                 u32* dup) {
+                                 IndexProbe* probe) {
     for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
          t += (i64)gridDim.x * blockDim.x) {
         other[t] = k[t] & 0xffffffffull;
         other32[t] = (u32)k[t];
         head[t] = (t == 0 || (k[t] >> 32) != (k[t - 1] >> 32)) ? 1u : 0u;
-        if (dup && t > 0 && k[t] == k[t - 1]) *dup = 1u;
+        if (probe && t > 0)
+            probe_pair(probe, k[t] >> 32, (u32)k[t], k[t - 1] >> 32, (u32)k[t - 1]);
     }
 }
 
@@ -206,18 +226,6 @@ int gsz(i64 n) {
     return (int)(b < 1 ? 1 : (b > 65535 ? 65535 : b));
 }
 
-// major 0: groups by alpha (companion beta); major 1: groups by beta.  With
-// n_orb <= 32 the sort runs on 64-bit keys over 32 + n_orb bits, and the
-// 32-bit companion strings of the scans come out of the same pass.
-// What the host reads of an index after its first phase: the group count,
-// the group lengths by floor(log2(len - 1)), and whether a determinant is
-// listed twice.
-struct IndexProbe {
-    u32 ngroups;
-    u32 dup;
-    u32 hist[32];
-};
-
 // First phase of a string index (no host synchronisation): sorted keys,
 // companions, group numbers and starts; the probe is filled on the device.
 // The sorted keys stay in X until str_index_finish.
@@ -229,7 +237,7 @@ void str_index_begin(StrIndex& X, const u64* V, i64 n, int major, int n_orb, Ind
     X.idx.alloc(n, s);
     X.other.alloc(n, s);
     DBuf<unsigned> head(n, s);
-    u32* dup = major == 0 ? &probe->dup : nullptr;
+    IndexProbe* pairs = major == 0 ? probe : nullptr;
     if (narrow) {
         k64.alloc(n, s);
         X.ks64.alloc(n, s);
@@ -238,7 +246,8 @@ void str_index_begin(StrIndex& X, const u64* V, i64 n, int major, int n_orb, Ind
         DNQ_CHECK_LAUNCH();
         const u64 mask[1] = {low_mask(n_orb) << 32 | low_mask(n_orb)};
         prim::radix_sort_masked<u64, u32>(k64.p, X.ks64.p, nullptr, X.idx.p, n, mask, s);
-        k_split_sorted64<<<gsz(n), 256, 0, s>>>(X.ks64.p, n, X.other.p, X.other32.p, head.p, dup);
+        k_split_sorted64<<<gsz(n), 256, 0, s>>>(X.ks64.p, n, X.other.p, X.other32.p, head.p,
+                                                  pairs);
         DNQ_CHECK_LAUNCH();
     } else {
         k.alloc(n, s);
@@ -247,7 +256,7 @@ void str_index_begin(StrIndex& X, const u64* V, i64 n, int major, int n_orb, Ind
         DNQ_CHECK_LAUNCH();
         const int bits[2] = {n_orb, n_orb};
         prim::radix_sort<ulonglong2, u32>(k.p, X.ks.p, nullptr, X.idx.p, n, bits, s);
-        k_split_sorted<<<gsz(n), 256, 0, s>>>(X.ks.p, n, X.other.p, head.p, dup);
+        k_split_sorted<<<gsz(n), 256, 0, s>>>(X.ks.p, n, X.other.p, head.p, pairs);
         DNQ_CHECK_LAUNCH();
     }
     X.gid.alloc(n, s);
@@ -292,10 +301,11 @@ void build_str_index(StrIndex& X, const u64* V, i64 n, int major, int n_orb, cud
     DBuf<IndexProbe> probe(1, s);
     DNQ_CUDA(cudaMemsetAsync(probe.p, 0, sizeof(IndexProbe), s));
     str_index_begin(X, V, n, major, n_orb, probe.p, s);
-    u32 ng = 0;
-    DNQ_CUDA(cudaMemcpyAsync(&ng, &probe.p->ngroups, 4, cudaMemcpyDeviceToHost, s));
+    IndexProbe hp;
+    DNQ_CUDA(cudaMemcpyAsync(&hp, probe.p, sizeof(hp), cudaMemcpyDeviceToHost, s));
     DNQ_CUDA(cudaStreamSynchronize(s));
-    str_index_finish(X, n, ng, s);
+    X.mixed = hp.mixed != 0;
+    str_index_finish(X, n, hp.ngroups, s);
 }
 
 __global__ void k_narrow(const u64* x, i64 n, u32* y) {
@@ -538,6 +548,7 @@ struct VVParams {
     double eps1;
     double cut;             // doubles: keep w >= cut (and > 1e-15)
     double single_thr;      // singles: keep |h| > single_thr
+    int mixed;              // several electron counts: matches need not be excitations
     const double* psi;
     u32 big_group;          // part C: binary search for groups longer than this
     int c_groupwalk;        // part C: short groups one at a time instead of packed
@@ -835,6 +846,7 @@ __device__ __forceinline__ Hit eval_hit(const VVParams& P, int r, u64 a, u64 b, 
         const u32 odd = (u32)between_w(s, lo, hi) ^ (tag >> 20);
         e.h = (odd & 1u) ? -raw : raw;
         e.keep = keep_double(cut, e.h);
+        if (P.mixed && popc_w((W)(s & x)) != 1) e.keep = false;
         e.j = j;
     } else if (kind == kHitD) {
         e.h = P.diag[r];
@@ -845,7 +857,9 @@ __device__ __forceinline__ Hit eval_hit(const VVParams& P, int r, u64 a, u64 b, 
         const W y = __ldg(&(alpha ? b_others<W>(P) : a_others<W>(P))[pos]);
         const W x = (W)(alpha ? a : b);
         const u32 j = __ldg(&(alpha ? P.b_idx : P.a_idx)[pos]);
-        if (popc_w((W)(x ^ y)) == 2) {
+        if (P.mixed && popc_w(x) != popc_w(y)) {
+            // not an excitation
+        } else if (popc_w((W)(x ^ y)) == 2) {
             e.h = str_single<W, AHEAD>(P, a, b, alpha ? 0 : 1, x, y);
             e.keep = keep_single(P, psr, e.h);
         } else {
@@ -1523,10 +1537,12 @@ __global__ void __launch_bounds__(256) k_vv_singles(Loc L, Arena A) {
         row_setup(P, r, a, b, psr, cut);
         const bool alpha = e.z == kHitA;   // the alpha string moves
         const u64 y = alpha ? __ldg(&P.b_other[e.y]) : __ldg(&P.a_other[e.y]);
-        const double h = str_single<u64>(P, a, b, alpha ? 0 : 1, alpha ? a : b, y);
-        SingleOut o;
-        o.h = h;
-        o.keep = keep_single(P, psr, h) ? 1u : 0u;
+        const u64 x = alpha ? a : b;
+        SingleOut o{0.0, 0u, 0u};
+        if (!P.mixed || __popcll(x) == __popcll(y)) {
+            o.h = str_single<u64>(P, a, b, alpha ? 0 : 1, x, y);
+            o.keep = keep_single(P, psr, o.h) ? 1u : 0u;
+        }
         o.j = alpha ? __ldg(&P.b_idx[e.y]) : __ldg(&P.a_idx[e.y]);
         A.sres[i] = o;
     }
@@ -2313,6 +2329,7 @@ VVParams make_params(dnq_ctx_s* ctx, const u64* V, i64 n, int n_orb, int policy,
     P.eps1 = eps1;
     P.cut = cut;
     P.single_thr = kElemThresh;
+    P.mixed = A.mixed;
     P.psi = psi;
     P.big_group = kBigGroup;
     P.c_groupwalk = opt.partc_groupwalk;
@@ -2402,6 +2419,7 @@ void build_vv_checked(dnq_ctx_s* ctx, const u64* V, i64 n, int n_orb, int policy
             "DetMap::from_ordered: duplicate determinant found");
     H->diag.alloc(n, s);
     launch_diag(ctx, V, n, H->diag.p, s);
+    A.mixed = hp[0].mixed != 0;
     str_index_finish(A, n, hp[0].ngroups, s);
     str_index_finish(B, n, hp[1].ngroups, s);
     build_presence_hist(A, B, n, hp[0].hist, s);
@@ -2638,16 +2656,6 @@ __global__ void k_sanitize(i64* rowptr, i64 n, i64 cap, const int* overflow, int
 constexpr u32 kSliceTests = 2048;        // tests per slice, few rows per warp
 constexpr u32 kSliceTestsMany = 1 << 17; // with many rows per warp only the longest are cut
 
-// Sets *mixed when the determinants differ in their electron counts (the
-// string tests count differing orbitals, which then says nothing of the
-// excitation rank).
-__global__ void k_mixed_counts(const u64* V, i64 n, u32* mixed) {
-    const int na = __popcll(V[0]), nb = __popcll(V[1]);
-    for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n;
-         t += (i64)gridDim.x * blockDim.x)
-        if (__popcll(V[2 * t]) != na || __popcll(V[2 * t + 1]) != nb) *mixed = 1u;
-}
-
 struct ContractOut {
     const double* coeff;
     DDb acc;
@@ -2789,18 +2797,12 @@ bool contract_strings(dnq_ctx_s* ctx, const u64* V, i64 n, const double* cd, int
     StrIndex A, B;
     str_index_begin(A, V, n, 0, n_orb, probe.p, s);
     str_index_begin(B, V, n, 1, n_orb, probe.p + 1, s);
-    DBuf<u32> mixed(1, s);
-    DNQ_CUDA(cudaMemsetAsync(mixed.p, 0, 4, s));
-    k_mixed_counts<<<gsz(n), 256, 0, s>>>(V, n, mixed.p);
-    DNQ_CHECK_LAUNCH();
     DBuf<double> diag(n, s);
     launch_diag(ctx, V, n, diag.p, s);
     IndexProbe hp[2];
-    u32 hmixed = 0;
     DNQ_CUDA(cudaMemcpyAsync(hp, probe.p, 2 * sizeof(IndexProbe), cudaMemcpyDeviceToHost, s));
-    DNQ_CUDA(cudaMemcpyAsync(&hmixed, mixed.p, 4, cudaMemcpyDeviceToHost, s));
     DNQ_CUDA(cudaStreamSynchronize(s));
-    if (hp[0].dup || hmixed) return false;
+    if (hp[0].dup || hp[0].mixed) return false;
     str_index_finish(A, n, hp[0].ngroups, s);
     str_index_finish(B, n, hp[1].ngroups, s);
     build_presence_hist(A, B, n, hp[0].hist, s);
