@@ -6,11 +6,12 @@
 //      H_PV = transpose (rows ascending inside each column, as coo_to_csc).
 //   2. D^-1 in FP64 (sigma: d/(d^2+eps^2), linear: 1/(d+sgn(d) eps)) and
 //      column screening |D^-1_k| * ||col_k||^2 < 1e-12 (ham_eff.cpp:93-106).
-//   3. One warp per output row i walks the entries (k, a) of H_VP row i in
-//      ascending k and scatters a*D^-1_k*H_VP[j,k] into a dense accumulator
-//      over j (shared memory when it fits, else a per-warp HBM slab), with a
-//      bitmap of touched columns; the k loop is sequential so every output
-//      element is summed in the reference's order.  FP64 mode uses
+//   3. One warp per output row i (or per half of its columns, k_heff) walks
+//      the entries (k, a) of H_VP row i in ascending k and scatters
+//      a*D^-1_k*H_VP[j,k] into a dense accumulator over j: in shared memory
+//      when it fits, else in a per-warp HBM slab with a bitmap of touched
+//      columns.  The k loop is sequential so every output element is summed in
+//      the reference's order.  FP64 mode uses
 //      unfused multiply/add like the reference build; FP32 mode reads FP32
 //      H_VP values and keeps a float-float accumulator per element: each
 //      product's rounding error (TwoProduct) and each sum's (TwoSum) go to
@@ -19,7 +20,7 @@
 //      accurate to a few FP32 ulps squared.
 //   4. The H_VV row is added, entries with |v| <= 1e-15 dropped
 //      (csr_add, ham_utils.cpp:330-442), and the row is compacted in column
-//      order from the bitmap.
+//      order: shared memory is swept whole, a slab by its bitmap.
 
 #include <memory>
 #include <type_traits>
@@ -242,9 +243,9 @@ __global__ void __launch_bounds__(kHW * 32) k_heff(HeffParams P) {
         const bool has_diag = i >= j0 && i < j1;
         // ---- scatter H_VP row i, k ascending.  Every H_PV column k of this
         // row holds row i itself, so the diagonal element receives one term
-        // per k: it is kept in lane 0's registers (same order of additions).
-        // The metadata of 32 k's is fetched at once by the lanes; columns
-        // that hold only row i need no slab access at all.
+        // per k: its sum is kept in registers, the same in every lane (same
+        // order of additions).  The metadata of 32 k's is fetched at once by the
+        // lanes; columns that hold only row i need no accumulator access at all.
         double dacc = 0.0;             // FP64 diagonal sum
         float dhi = 0.0f, dlo = 0.0f;  // FP32 float-float diagonal sum
         bool dtouch = false;
@@ -1107,7 +1108,12 @@ void ham_eff_csr(const Csr& VV, const Csr& VP, i64 nv, i64 np, const double* hpp
     DNQ_CHECK_LAUNCH();
     // Accumulators in shared memory for up to 6,400 rows; halves where the
     // columns average more than 24 entries (one step is 32): 1.61 -> 1.49 ms at
-    // 30 entries, while shorter columns would only have their metadata read twice
+    // 2,241 rows of a 13-orbital space (30 entries).  On 2e6 random entries, one unit
+    // a row and two (FP64, us): columns of 25, 43 and 85 entries 981 and 902, 1419
+    // and 1212, 2253 and 1453 at 500 rows; 423 and 324, 633 and 440, 931 and 663 at
+    // 2,241; 954 and 586, 1342 and 784, 1909 and 1091 at 6,000.  Shorter columns
+    // have their metadata read twice: 7 entries 868 and 886 at 500 rows, but 402 and
+    // 320 at 2,241, where the smaller accumulators let more warps in.
     constexpr size_t kSmem = 200 * 1024;
     const bool smem = (size_t)nv * 8 * kHW <= kSmem;
     const int halves = smem && nv >= 64 && VP.nnz > 24 * np ? 2 : 1;

@@ -320,7 +320,9 @@ void spmm_g(int G, int U, const Csr& m, const T* val, const T* Xg, const double*
 #undef DNQ_SPMM_U
 }
 
-constexpr int kEnergyBlocks = 592;   // the single-vector reduction's grid
+// The most blocks of the single-vector reduction (it launches fewer for short
+// vectors; the partials of blocks without rows are zero and change no sum).
+constexpr int kEnergyBlocks = 592;
 
 }  // namespace
 

@@ -24,9 +24,11 @@
 // records their members in warp-private arena chunks (single excitations
 // also in a per-warp list), k_vv_singles evaluates the singles one per
 // thread, k_vv_eval turns each row's members into entries in place,
-// k_vv_big / k_vv_eval_long / k_vv_compact_long handle rows longer than a
-// chunk, and k_vv_compact gathers the CSR.  k_vv_twopass is the exact
-// fallback when the arena runs out.
+// k_vv_big / k_vv_eval_long and k_vv_long_inplace (k_vv_compact_long in
+// batches) handle the long rows -- those that overflow a chunk, and those of
+// more than kLongEval members and twice a warp's share of all members --, and
+// k_vv_compact gathers a batch's CSR.  k_vv_twopass is the exact fallback when
+// the arena runs out.
 
 #include <algorithm>
 #include <type_traits>
@@ -594,7 +596,7 @@ struct Arena {
     int* overflow;                    // set when the arena is too small
     i64* row_pos;
     u32* row_len;
-    u32* big;                         // rows longer than one chunk
+    u32* big;                         // long rows (past a chunk, or listed by k_vv_eval)
     u32* big_len;                     // their member counts
     int* n_big;
     uint2* unit;                      // 64-member units of the long rows: (place in big, unit)
@@ -2788,8 +2790,8 @@ __global__ void __launch_bounds__(256) k_contract_final(const double2* epart, in
 
 // E (and sigma, optional) by string groups.  False when the basis lists a
 // determinant twice (its amplitudes then follow the de-duplicated order,
-// which the candidate walk's map holds) or mixes electron counts.  Host synchronisations: the sizes of
-// the indices, the slice count and the result.
+// which the candidate walk's map holds) or mixes electron counts.  Host
+// synchronisations: the sizes of the indices, the slice count and the result.
 bool contract_strings(dnq_ctx_s* ctx, const u64* V, i64 n, const double* cd, int n_orb,
                       double single_thr, double cut, double* sigma, cudaStream_t s, double* e) {
     DBuf<IndexProbe> probe(2, s);

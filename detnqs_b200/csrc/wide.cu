@@ -248,8 +248,9 @@ __device__ __forceinline__ DiagTab stage_diag_tab(const CtxView& C, double* mem)
     return DiagTab{mem, mem + n, mem + n + nn, n};
 }
 
-// diag2 from staged tables: occupied orbitals listed four to a word, so that a pair costs an extraction, a table read and an
-// addition and four reads are in flight.  The same additions in the same order.
+// diag2 from staged tables: occupied orbitals listed four to a word, so that a
+// pair costs an extraction, a table read and an addition and four reads are in
+// flight.  The same additions in the same order.
 //
 // Bound: issue slots (74% with the orbitals found bit by bit, where 4.2e6
 // determinants of 100 orbitals and 40 electrons took 1.69 ms; 2.20 with one
