@@ -33,7 +33,7 @@ struct SlotPool {
     // is made only where it can be kept, and once the plain copies have cost as
     // much.
     char* take(size_t n) {
-        std::lock_guard<std::mutex> lk(mu);
+        std::unique_lock<std::mutex> lk(mu);
         for (auto& p : kept)
             if (p) {
                 char* q = p;
@@ -43,13 +43,15 @@ struct SlotPool {
         if (contexts == 0 || made == kKept) return nullptr;
         plain += n;
         if (plain < kWorth) return nullptr;
-        void* q = nullptr;
-        if (cudaHostAlloc(&q, kSlots, cudaHostAllocPortable) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return nullptr;   // no page-locked memory
-        }
         ++made;
-        return static_cast<char*>(q);
+        lk.unlock();   // other copies and contexts do not wait for the driver
+        void* q = nullptr;
+        if (cudaHostAlloc(&q, kSlots, cudaHostAllocPortable) == cudaSuccess)
+            return static_cast<char*>(q);
+        (void)cudaGetLastError();
+        lk.lock();
+        --made;
+        return nullptr;   // no page-locked memory
     }
     void give(char* q) noexcept {
         {
