@@ -78,3 +78,28 @@ def test_energy_and_pt2(space, use_hb):
     assert got["n_ext"] == want["n_ext"]
     for part in ("e_pt2_external", "e_pt2_internal"):
         assert abs(got[part] - want[part]) <= 1e-12 * max(1.0, abs(want[part]))
+
+
+# large enough for the string groups (builds of V alone, energy, batch), in
+# one word and in two
+@pytest.mark.parametrize("n,n_orb", [(20, 16), (36, 33)])
+def test_string_groups(port, n, n_orb):
+    from detnqs_b200 import core, native as N
+    from detnqs_b200.batch import Batch
+    sysm = S.make_system(n, 4, 4, 2 * n, 3)
+    V = np.ascontiguousarray(S.hf_sd_space(n_orb, 4, 4)[:2500])
+    psi = S.normalized_psi(len(V), 1)
+    ctx = core.IntCtx.from_arrays(n, sysm.h1e, sysm.eri, sysm.e_core)
+    ctx.hb_prepare(1e-15)
+    octx = port.ctx_from_arrays(n, sysm.h1e, sysm.eri, sysm.e_core)
+    octx.hb_prepare(1e-15)
+    octx.n_orb = n_orb
+    want = octx.get_ham_vv(V)
+    assert_coo_equal(core.get_ham_vv(V, ctx, n_orb), want)
+    b = Batch([ctx], [V], [n_orb], policy=N.POLICY_KNOWN_SETS, use_heatbath=False, eps1=0.0)
+    assert_coo_equal(b.coo(0), want)
+    b.close()
+    e = core.compute_variational_energy(V, psi, ctx, n_orb, True, 1e-5)
+    e0 = octx.compute_variational_energy(V, psi, True, 1e-5)
+    assert abs(e - e0) <= 1e-12 * max(1.0, abs(e0))
+    ctx.close()
