@@ -38,8 +38,8 @@ void set_last_error(const std::string& msg);
     do {                                                                      \
         cudaError_t _e = (call);                                              \
         if (_e != cudaSuccess) {                                              \
+            (void)cudaGetLastError();   /* not for the next launch's check */ \
             if (_e == cudaErrorMemoryAllocation) {                            \
-                (void)cudaGetLastError();                                     \
                 throw ::dnq::Error(DNQ_ERR_OUT_OF_MEMORY,                     \
                                    std::string("out of device memory at ") +  \
                                        #call);                                \
