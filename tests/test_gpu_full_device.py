@@ -2,6 +2,8 @@
 pool's unused pieces: the arena shrinks and the two-pass walk builds the
 block."""
 
+import contextlib
+
 import numpy as np
 import pytest
 
@@ -13,44 +15,42 @@ MB = 1 << 20
 LEFT = 192 * MB   # to be left free; the whole arena of this build takes 350 MB
 
 
-class _Full:
+@contextlib.contextmanager
+def _full():
     """The device's pool with 15 MB holes (more than an arena in all) between
     pieces in use, and the device filled up to LEFT."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
 
-    def __enter__(self):
-        self.rt = rt = pytest.importorskip("cuda.bindings.runtime")
-        self.pieces, self.fill = [], []
+    def ok(r):
+        assert r[0] == rt.cudaError_t.cudaSuccess, r
+        return r[1] if len(r) > 1 else None
 
-        def ok(r):
-            assert r[0] == rt.cudaError_t.cudaSuccess, r
-            return r[1] if len(r) > 1 else None
-
-        self.ok = ok
-        self.pool = ok(rt.cudaDeviceGetDefaultMemPool(0))
-        ok(rt.cudaDeviceSynchronize())
-        ok(rt.cudaMemPoolTrimTo(self.pool, 0))
-        self.pieces = [ok(rt.cudaMallocAsync(MB, 0)) for _ in range(1024)]
-        for k, p in enumerate(self.pieces):
-            if k % 16:
-                ok(rt.cudaFreeAsync(p, 0))
-        self.pieces = self.pieces[::16]
+    pool = ok(rt.cudaDeviceGetDefaultMemPool(0))
+    ok(rt.cudaDeviceSynchronize())
+    ok(rt.cudaMemPoolTrimTo(pool, 0))
+    pieces, fill = [], []
+    try:
+        for _ in range(1024):
+            pieces.append(ok(rt.cudaMallocAsync(MB, 0)))
+        for p in [p for k, p in enumerate(pieces) if k % 16]:
+            pieces.remove(p)
+            ok(rt.cudaFreeAsync(p, 0))
         ok(rt.cudaDeviceSynchronize())
         size = 64 << 30
         while size >= 8 * MB:
             free = rt.cudaMemGetInfo()[1]
             if free - size >= LEFT:
-                self.fill.append(ok(rt.cudaMalloc(size)))
+                fill.append(ok(rt.cudaMalloc(size)))
             else:
                 size //= 2
-        return self
-
-    def __exit__(self, *exc):
-        for p in self.fill:
-            self.ok(self.rt.cudaFree(p))
-        for p in self.pieces:
-            self.ok(self.rt.cudaFreeAsync(p, 0))
-        self.ok(self.rt.cudaDeviceSynchronize())
-        self.ok(self.rt.cudaMemPoolTrimTo(self.pool, 0))
+        yield
+    finally:
+        for p in fill:
+            rt.cudaFree(p)
+        for p in pieces:
+            rt.cudaFreeAsync(p, 0)
+        ok(rt.cudaDeviceSynchronize())
+        ok(rt.cudaMemPoolTrimTo(pool, 0))
 
 
 def test_build_in_scattered_memory():
@@ -75,7 +75,7 @@ def test_build_in_scattered_memory():
         block()
     finally:
         N.check(N.lib.dnq_set_option(N.OPT_ARENA_CAP, 0))
-    with _Full():
+    with _full():
         got = block()
     for key in ("row", "col", "val"):
         np.testing.assert_array_equal(got[key].view(np.uint8), want[key].view(np.uint8))
